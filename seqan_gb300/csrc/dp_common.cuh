@@ -101,8 +101,6 @@ struct TraceArgs {
     int32_t local;
     int32_t band_w;        // banded layout: slots per column (0: not banded)
     int32_t band_upper;
-    int32_t warp_rows;     // warp layout: rows per lane strip (0: not the warp layout)
-    int32_t warp2;         // 1: the packed 16-bit warp layout with 4-bit cells (dp_warp2_kernels.cuh)
     int32_t dynamic;       // 1: DynamicGaps cells; best_e holds the best cell's gap flags
     int32_t extend;        // 1: AlignExtend_ (TraceHead_ but no TraceTail_, align_extend_base.h:67-73)
 };

@@ -70,21 +70,31 @@ __host__ __device__ inline int64_t warp2_trace_bytes(int m, int n)
     return warp2_band_off(m, bands - 1) + int64_t(m + 64) * 32 * warp2_last_rows(n);
 }
 
+// Byte offset of the trace word that holds cell (col, row) within the pair's trace (row 0: the
+// cell's byte).
+__device__ __forceinline__ int64_t trace_off_warp2(int m, int n, int col, int row)
+{
+    if (row == 0) return col;
+    const int r0 = row - 1;
+    const int b = r0 / kW2BandRows;
+    const int Rb = (b == (n - 1) / kW2BandRows) ? warp2_last_rows(n) : kW2Rows;
+    const int s = (r0 - b * kW2BandRows) / Rb;
+    return warp2_band_off(m, b) + (int64_t(col + s) * 32 + (s & 31)) * Rb;
+}
+
 // TraceBitMap_ byte of cell (col, row) from the 4-bit planes.
 __device__ __forceinline__ uint8_t trace_at_warp2(const uint8_t *base, int m, int n, bool affine, int col, int row)
 {
-    if (row == 0) return base[col];
+    const uint8_t *w = base + trace_off_warp2(m, n, col, row);
+    if (row == 0) return *w;
     const int r0 = row - 1;
     const int b = r0 / kW2BandRows;
     const int Rb = (b == (n - 1) / kW2BandRows) ? warp2_last_rows(n) : kW2Rows;
     const int within = r0 - b * kW2BandRows;
     const int s = within / Rb, r = within - s * Rb;
-    const int lane = s & 31, h = s >> 5;
-    const int t = col + lane + 32 * h;
-    const uint8_t *w = base + warp2_band_off(m, b) + (int64_t(t) * 32 + lane) * Rb;
     const uint32_t word = Rb == 4 ? *reinterpret_cast<const uint32_t *>(w)
                                   : (Rb == 2 ? uint32_t(*reinterpret_cast<const uint16_t *>(w)) : uint32_t(*w));
-    const int sh = h * 4 * Rb + r;
+    const int sh = (s >> 5) * 4 * Rb + r;
     const int b0 = (word >> sh) & 1, b1 = (word >> (sh + Rb)) & 1;
     const int eo = (word >> (sh + 2 * Rb)) & 1, fo = (word >> (sh + 3 * Rb)) & 1;
     if (b1 && !b0) return TV_NONE;

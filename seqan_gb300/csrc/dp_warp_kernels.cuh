@@ -84,17 +84,16 @@ __host__ __device__ inline int64_t warp_band_trace_off(int m, int b, int R)
     return align16(m + 1) + int64_t(b) * (m + 32) * 32 * R;
 }
 
-__device__ __forceinline__ uint8_t trace_at_warp(const uint8_t *base, int m, int n, int R, int col, int row)
+// Byte offset of the trace of cell (col, row) within the pair's trace.
+__device__ __forceinline__ int64_t trace_off_warp(int m, int n, int R, int col, int row)
 {
-    if (row == 0) return base[col];
+    if (row == 0) return col;
     const int r0 = row - 1;
     const int b = r0 / (32 * R);
     const int Rb = (b == (n - 1) / (32 * R)) ? warp_last_rows(n, R) : R;
     const int within = r0 - b * 32 * R;
-    const int lane = within / Rb;
-    const int r = within - lane * Rb;
-    const int t = col + lane;
-    return base[warp_band_trace_off(m, b, R) + (int64_t(t) * 32 + lane) * Rb + r];
+    const int t = col + within / Rb;
+    return warp_band_trace_off(m, b, R) + int64_t(t) * 32 * Rb + within;
 }
 
 struct WarpBest {

@@ -128,7 +128,6 @@ struct gba_plan {
     std::vector<int64_t> w2b_start, w2b_count;   // plain form: task ranges per length bucket
     int64_t num_warp_tasks = 0;     // (pair, band) work items
     int64_t num_band_states = 0;    // bands of pairs that span more than one band
-    int64_t num_tiled_tb = 0;       // leading slots whose traceback a whole warp walks
     int64_t grid16[8] = {};         // resident blocks of each packed-kernel variant
     int variant16 = 0;              // chosen tiling variant
     bool tune_pending = false;      // autotune at the first run
@@ -803,14 +802,6 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
         trace_off = wsize[nw];
         plan->trace_total = trace_off;
     }
-    // Large pairs of the warp layout (a prefix of the cost-sorted order) get the warp-walked
-    // traceback; the key is strips of STRIP_ROWS rows x (m + 1) columns.
-    plan->num_tiled_tb = 0;
-    if (plan->use_warp && plan->traceback && !(p->flags & GBA_FLAG_PLAIN_BUCKETS))
-        while (plan->num_tiled_tb < int64_t(keys.size()) &&
-               keys[plan->num_tiled_tb] >= uint32_t(kTiledTraceCells / STRIP_ROWS))
-            ++plan->num_tiled_tb;
-
     // Packed path: neighbours in the length-sorted order share a thread; per warp, the code
     // words (4 residues per word, both pairs' codes per byte) and the boundary row are
     // interleaved by lane.
@@ -1309,6 +1300,9 @@ __global__ void k_fill_invalid(const PairDesc *pairs, int64_t n, int32_t minval,
     if (cig_count) cig_count[k] = 0;
 }
 
+// Blocks of a kernel that gives each of `warps` items a warp.
+int warp_blocks(int64_t warps) { return int((warps * 32 + kBlock - 1) / kBlock); }
+
 // Enqueues the kernels of a plan on device inputs.  Scores/end positions go to the given
 // device pointers; segments and CIGARs stay in the plan's device buffers.
 int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const uint8_t *dseq_v,
@@ -1590,23 +1584,12 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
             t.extend = plan->extend;
             t.band_w = plan->params.band_on ? plan->params.band_upper - plan->params.band_lower + 1 : 0;
             t.band_upper = plan->params.band_upper;
-            t.warp_rows = plan->use_warp ? plan->warp_rows : 0;
-            t.warp2 = 0;
             t.dynamic = plan->dynamic;
-            const int64_t L = plan->num_tiled_tb;
-            if (L > 0) {
-                TraceArgs tl = t;
-                tl.num_slots = L;
-                k_traceback_tiled<kWarpRows><<<int((L + 1) / 2), 64, 0, ctx->stream>>>(tl);
-                ++launches;
-            }
-            if (plan->num_slots > L) {
-                TraceArgs ts = t;
-                ts.order = t.order + L;
-                ts.num_slots = plan->num_slots - L;
-                k_traceback<<<int((ts.num_slots + kBlock - 1) / kBlock), kBlock, 0, ctx->stream>>>(ts);
-                ++launches;
-            }
+            if (plan->use_warp)
+                k_traceback_warp<false, kWarpRows><<<warp_blocks(plan->num_slots), kBlock, 0, ctx->stream>>>(t);
+            else
+                k_traceback<<<int((plan->num_slots + kBlock - 1) / kBlock), kBlock, 0, ctx->stream>>>(t);
+            ++launches;
             GBA_CUDA(ctx, cudaGetLastError());
         }
         if (plan->num_w2 > 0) {
@@ -1630,8 +1613,7 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
             t.num_slots = plan->num_w2;
             t.affine = plan->affine;
             t.local = plan->local;
-            t.warp2 = 1;
-            k_traceback<<<int((plan->num_w2 + kBlock - 1) / kBlock), kBlock, 0, ctx->stream>>>(t);
+            k_traceback_warp<true, kW2Rows><<<warp_blocks(plan->num_w2), kBlock, 0, ctx->stream>>>(t);
             ++launches;
             GBA_CUDA(ctx, cudaGetLastError());
         }
