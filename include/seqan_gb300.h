@@ -122,11 +122,11 @@ typedef struct {
  * With equality scoring the engine uses its packed two-pairs-per-thread 16-bit kernel for global
  * score-only pairs when alphabet_size is between 1 and 8 (the caller's promise that every code is
  * below it, as the reference's alphabet types guarantee), the pair's values stay in the exact
- * int16 range and the batch holds at least 32768 pairs.  Other unbanded pairs with 16-bit cells in
- * the exact range, fewer than 1024 columns and at most 4096 rows, in batches of at least 4096
- * pairs, run the packed 16-bit warp kernel (two strips per lane, 4-bit trace; equality scoring
- * needs alphabet_size 1..8 there too); the remaining unbanded pairs run the 32-bit warp kernel,
- * banded pairs one thread per pair. */
+ * int16 range and the batch holds at least 32768 pairs.  Other unbanded pairs whose values fit 16
+ * bits (gap scores from -1024 to 0, every score between about -31,600 and 32,700) run the packed
+ * 16-bit warp kernel (two strips per lane; equality scoring needs alphabet_size 1..8 there too), with
+ * 16- and 32-bit score types alike; the remaining unbanded pairs run the 32-bit warp kernel, banded
+ * pairs one thread per pair. */
 enum {
     GBA_FLAG_GENERAL_KERNEL = 1,   /* force the one-pair-per-thread 32-bit kernel */
     GBA_FLAG_STRIP16 = 2,          /* packed kernel with 16-row strips instead of 32 */
@@ -145,8 +145,9 @@ enum {
     GBA_FLAG_PACKED_NO_SPLIT = 128,/* packed kernel: no split slots (two pairs per thread only) */
     GBA_FLAG_NO_WARP16 = 256,      /* pairs the packed 16-bit warp kernel would take run on the
                                       32-bit warp kernel instead */
-    GBA_FLAG_WARP16 = 512,         /* packed 16-bit warp kernel for eligible pairs even in batches
-                                      smaller than 4096 pairs */
+    GBA_FLAG_WARP16 = 512,         /* packed 16-bit warp kernel only for pairs with 16-bit cells in the
+                                      exact int16 range, fewer than 1024 columns and at most 4096
+                                      rows; the others run the 32-bit warp kernel */
     /* Not a kernel selection: GBA_ALIGN_EXTEND's X-drop terminator, threshold gba_params.xdrop. */
     GBA_FLAG_XDROP = 1024
 };

@@ -55,7 +55,8 @@ struct PairDesc {
     int32_t m;           // |H| (columns)
     int32_t n;           // |V| (rows)
     int32_t inf;         // DPCellDefaultInfinity of the cell width the pair runs with
-    int32_t invalid;     // 1: empty sequence or band outside the matrix (score = numeric min)
+    int16_t invalid;     // 1: empty sequence or band outside the matrix (score = numeric min)
+    int16_t rows;        // packed 16-bit warp kernel: rows per strip
 };
 
 // Arguments of the DP kernels, passed by value.

@@ -13,6 +13,7 @@
 #include "dp_banded_kernels.cuh"
 #include "dp_warp_kernels.cuh"
 #include "dp_warp2_kernels.cuh"
+#include "warp2_launch.cuh"
 #include "dp_dynamic_kernels.cuh"
 #include "seed_kernels.cuh"
 #include "extend_kernels.cuh"
@@ -122,6 +123,9 @@ struct gba_plan {
     int64_t num_w2 = 0;             // pairs
     int64_t num_w2_tasks = 0;       // (pair, band) tasks
     int64_t num_w2_states = 0;      // bands of pipelined pairs
+    int64_t num_w2_entries = 0;     // row buffer entries
+    int w2_mat = 0;                 // W2_EQUAL / W2_PROFILE / W2_TABLE
+    size_t w2_smem = 0;             // dynamic shared memory of a block
     int64_t grid_w2 = 0;
     DevBuf tasks_w2, order_w2, rowbuf_w2, rowbuf_w2_off, counter_w2, band_w2, band_w2_base;
     std::vector<int2> h_w2tasks;
@@ -198,8 +202,9 @@ struct gba_plan {
 
 struct gba_context {
     std::map<int64_t, int> tuning;  // batch shape -> packed-kernel variant (autotuner results)
-    std::map<const void *, int64_t> grid_cache;   // kernel -> resident blocks on this device
+    std::map<std::pair<const void *, size_t>, int64_t> grid_cache;   // (kernel, shared memory) -> resident blocks
     int device = 0;
+    int sms = 0;                    // device_sms
     int64_t budget = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[6] = {};
@@ -278,12 +283,9 @@ constexpr int64_t kChunkPairs = 200000;
 // Pairs at least this wide pipeline their bands across warps even in large batches: the ~130
 // steps a pipelined band waits before its first column are then a small share of its work.
 constexpr int kPipelineMinCols = 1024;
-// The packed 16-bit warp kernel takes pairs narrower than kPipelineMinCols with at most kW2MaxRows
-// rows, in batches of at least kW2MinPairs pairs (it runs each pair's bands in order on one warp).
+// GBA_FLAG_WARP16 keeps the packed 16-bit warp kernel to pairs of the exact int16 range with fewer
+// than kPipelineMinCols columns and at most kW2MaxRows rows.
 constexpr int kW2MaxRows = 4096;
-// Pairs of at least this many 256-row bands pipeline their bands across warps.
-constexpr int kW2PipeBands = 3;
-constexpr int64_t kW2MinPairs = 4096;
 
 // _checkBandProperties (align/dp_algorithm_impl.h:193-234): the band must meet the matrix and
 // may leave it only across sides whose end gaps are free.
@@ -346,6 +348,37 @@ bool int16_exact(const gba_params &p, int max_pos, int64_t m, int64_t n, bool lo
     if (local) return true;
     const int64_t lower = -(3 * open + ext * (m + n + 2));
     return lower > -16384 + 2 * (open + ext) + 64;
+}
+
+// True when the packed 16-bit warp kernel's arithmetic gives an m x n pair's exact values: every
+// value a real cell takes lies between its "infinity" and 32767.  Scores are bounded as in
+// int16_exact, with 64 columns more: a strip's lanes run on past the last column, and their halves
+// must not carry into their neighbours.  Gap scores are at most 0 (build_plan).
+bool w2_fits(const gba_params &p, int max_pos, int64_t m, int64_t n, bool local)
+{
+    const int64_t open = -int64_t(p.gap_open), ext = -int64_t(p.gap_extend);
+    if (int64_t(max_pos) * (std::min(m, n) + 64) > 32767 - 64) return false;
+    return local || -(3 * open + ext * (m + n + 66)) > kW2Inf + 2 * (open + ext) + 64;
+}
+
+// Rows per strip (2, 3, 4, 5, 6 or 8) that cover n rows in `bands` bands.
+int w2_rows(int64_t n, int bands, int most)
+{
+    const int r = int((n + 64 * int64_t(bands) - 1) / (64 * int64_t(bands)));
+    return r <= 2 ? 2 : (r == 7 ? std::min(8, most) : r);
+}
+
+// Nanoseconds of an SM sub-partition for an m x n pair with R rows per strip when enough warps share
+// it (w2_busy), and until the pair is done when its bands have the device to themselves, in order on
+// one warp or pipelined over one warp each (w2_alone).  Fitted to GB300 measurements of the affine
+// kernel at 40 to 10,000 bp: a lone warp waits on its own instructions, so a step's fixed part (hand-off,
+// loop) weighs five rows there and one and a half otherwise; a pipelined band starts about 90 steps
+// behind the one above (63 of the front, kW2Chunk read ahead, and the trip of an entry through L2).
+double w2_busy(int64_t m, int64_t n, int R) { return w2_bands(int(n), R) * double(m + 64) * (27 + 18 * R); }
+double w2_alone(int64_t m, int64_t n, int R, bool pipelined)
+{
+    const double bands = w2_bands(int(n), R), steps = pipelined ? m + 64 + 90 * (bands - 1) : bands * (m + 64);
+    return steps * (85 + 17 * R);
 }
 
 int validate(gba_context *ctx, const gba_params *p, const gba_batch *b)
@@ -514,23 +547,32 @@ void launch_dp16(int v, bool affine, int grid, const Dp16Args &a, cudaStream_t s
 #undef GBA_L16
 }
 
+int device_sms(gba_context *ctx)
+{
+    if (ctx->sms == 0) cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    return ctx->sms > 0 ? ctx->sms : 1;
+}
+
 // Resident blocks of a persistent kernel on this device (all SMs x blocks per SM); the
 // occupancy queries are cached per context (they do not change).
-int64_t persistent_grid(gba_context *ctx, const void *fn)
+int64_t persistent_grid(gba_context *ctx, const void *fn, size_t smem = 0)
 {
-    auto it = ctx->grid_cache.find(fn);
+    auto it = ctx->grid_cache.find({fn, smem});
     if (it != ctx->grid_cache.end()) return it->second;
-    int sms = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, 0) != cudaSuccess || per_sm < 1)
+    int per_sm = 0;
+    // One limit for every alphabet (a smaller one set later would refuse the larger launches).
+    if (smem > 0)
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             int(std::max(smem, w2_shared_bytes(W2_PROFILE, 32))));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kBlock, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const int64_t g = int64_t(sms) * per_sm;
-    ctx->grid_cache.emplace(fn, g);
+    const int64_t g = int64_t(device_sms(ctx)) * per_sm;
+    ctx->grid_cache.emplace(std::make_pair(fn, smem), g);
     return g;
 }
 
 const void *warp_fn(bool a, bool l, bool m, bool t);
-const void *warp2_fn(bool a, bool l, bool m, bool t);
+Warp2Fn warp2_fn(bool a, bool l, int mat, bool t);
 
 // Host threads for a planning loop over `work` items: serial below 16,384 items.
 int plan_threads(int64_t work)
@@ -604,18 +646,24 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     // one-pair-per-thread kernel is forced.
     plan->use_warp = !p->band_on && !(p->flags & GBA_FLAG_GENERAL_KERNEL) && !plan->dynamic;
     plan->warp_rows = 8;
-    // The packed 16-bit warp path: 16-bit cells, a batch large enough to fill the GPU with one
-    // warp per pair, equality scoring over at most 8 codes (PRMT lookup) or a table whose entries
-    // fit int16, and gap scores small enough for the int16 range checks.
-    bool w2_ok = plan->use_warp && p->score_bits == 16 && (N >= kW2MinPairs || (p->flags & GBA_FLAG_WARP16)) &&
-                 !(p->flags & GBA_FLAG_NO_WARP16) &&
-                 std::abs(p->gap_open) <= 1024 && std::abs(p->gap_extend) <= 1024;
+    // The packed 16-bit warp path: equality scoring over at most 8 codes (PRMT lookup), a table whose
+    // entries fit a byte (score profile) or at most 1024 (table lookup), and gap scores small enough
+    // for its 16-bit arithmetic; each pair's range is checked below.
+    bool w2_ok = plan->use_warp && !(p->flags & GBA_FLAG_NO_WARP16) && p->gap_open <= 0 && p->gap_extend <= 0 &&
+                 p->gap_open >= -1024 && p->gap_extend >= -1024;
+    plan->w2_mat = W2_EQUAL;
     if (w2_ok && plan->matrix) {
-        for (int32_t v : plan->matrix_host) w2_ok = w2_ok && v >= -1024 && v <= 1024;
+        plan->w2_mat = W2_PROFILE;
+        for (int32_t v : plan->matrix_host) {
+            w2_ok = w2_ok && v >= -1024 && v <= 1024;
+            if (v < -128 || v > 127) plan->w2_mat = W2_TABLE;
+        }
     } else if (w2_ok) {
         w2_ok = p->alphabet_size >= 1 && p->alphabet_size <= 8 && p->match >= -128 && p->match <= 127 &&
                 p->mismatch >= -128 && p->mismatch <= 127;
     }
+    const bool w2_narrow = (p->flags & GBA_FLAG_WARP16) != 0;
+    const int w2_most = w2_max_rows(plan->w2_mat, plan->local, plan->traceback);
     // Host arrays live in the plan and keep their capacity between builds (no zero fill).
     auto &keys16 = plan->h_keys16;
     auto &idx16 = plan->h_idx16;
@@ -645,8 +693,9 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     std::vector<int64_t> c16(nth + 1, 0), cot(nth + 1, 0), ctr(nth + 1, 0), cw2(nth + 1, 0);
     int64_t first_bad = N, cells = 0;
     double cells16 = 0;   // cells of the packed-path pairs
+    double cost2 = 0;     // steps x instructions of the packed warp path's pairs
     const int fe_all = plan->local ? 15 : plan->free_ends;
-#pragma omp parallel num_threads(nth) reduction(+ : cells, cells16) reduction(min : first_bad)
+#pragma omp parallel num_threads(nth) reduction(+ : cells, cells16, cost2) reduction(min : first_bad)
     {
         const int t = omp_get_thread_num();
         const int64_t k0 = N * t / nth, k1 = N * (t + 1) / nth;
@@ -669,6 +718,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
             d.n = int32_t(v1 - v0);
             d.trace_off = 0;
             d.invalid = 0;
+            d.rows = 0;
             const bool exact16 = p->score_bits == 16 && int16_exact(*p, max_pos, d.m, d.n, plan->local);
             d.inf = exact16 ? -16384 : -(1 << 30);
             plan->status[k] = (p->score_bits == 16 && !exact16) ? GBA_PAIR_PROMOTED : GBA_PAIR_OK;
@@ -693,9 +743,12 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
                 cls[k] = 1;
                 ++n16;
                 cells16 += double(d.m) * d.n;
-            } else if (w2_ok && exact16 && d.m < kPipelineMinCols && d.n <= kW2MaxRows) {
-                const int64_t bands = (d.n + kW2BandRows - 1) / kW2BandRows;
-                key[k] = uint32_t(std::min<int64_t>(bands * (d.m + 64), 0xffffffffLL));
+            } else if (w2_ok && w2_fits(*p, max_pos, d.m, d.n, plan->local) &&
+                       (!w2_narrow || (p->score_bits == 16 && exact16 && d.m < kPipelineMinCols && d.n <= kW2MaxRows))) {
+                d.rows = int16_t(w2_rows(d.n, w2_bands(d.n, w2_most), w2_most));
+                const double c = w2_busy(d.m, d.n, d.rows);
+                cost2 += c;
+                key[k] = uint32_t(std::min<double>(c / 64, 4e9));
                 cls[k] = 3;
                 ++nw2;
             } else {
@@ -706,7 +759,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
             }
             if (plan->traceback) {
                 tbytes[k] = p->band_on ? int64_t(d.m + 1) * band_col_bytes(p->band_upper - p->band_lower + 1) / 32
-                            : cls[k] == 3 ? warp2_trace_bytes(d.m, d.n)
+                            : cls[k] == 3 ? w2_trace_bytes(d.m, d.n, d.rows, plan->local)
                             : plan->use_warp ? warp_trace_bytes(d.m, d.n, plan->warp_rows)
                                              : trace_bytes(d.m, d.n);
                 tsum += tbytes[k];
@@ -984,19 +1037,28 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
         sort_desc(keys2, idx2);
     }
     plan->num_w2 = int64_t(idx2.size());
-    // Tasks: (pair, -1) runs the pair's bands in order on one warp; a pair of at least
-    // kW2PipeBands bands, or of two or more in a batch too small to keep the GPU busy otherwise,
-    // becomes one task per band, pipelined across warps.  Row buffers: one slot of m + 1 words for
-    // in-order pairs, two for pipelined ones; pipelined bands get a BandState each.
+    // Tasks: (pair, -1) runs the pair's bands in order on one warp; a pair that would keep its warp
+    // busy for longer than a quarter of what the whole batch takes on the device becomes one task per
+    // band, pipelined across warps, if that ends a fifth sooner, with fewer rows per strip (more bands
+    // at once) the longer it is: the most rows whose pipeline ends within that quarter, else the rows
+    // that end first.  Measured on 2,000 pairs of 100 to 10,000 bp (DP alone): an eighth 4.94 ms, a
+    // quarter 4.47, half 4.96, all of it 6.79.  The plain form pipelines bands only in batches too small to keep the GPU busy otherwise.  Row buffers: one
+    // slot of m + 1 entries for in-order pairs, two for pipelined ones; pipelined bands get a
+    // BandState each.
     std::vector<int64_t> rb2off, bs2base;
     std::vector<int2> &w2tasks = plan->h_w2tasks;
     w2tasks.clear();
     int64_t rb2tot = 0, ns2 = 0;
     if (plan->num_w2 > 0) {
-        plan->grid_w2 = persistent_grid(ctx, warp2_fn(plan->affine, plan->local, plan->matrix, plan->traceback));
-        const bool few = plan->num_w2 < 2 * plan->grid_w2 * (kBlock / 32);
+        const Warp2Fn fn = warp2_fn(plan->affine, plan->local, plan->w2_mat, plan->traceback);
+        plan->w2_smem = w2_shared_bytes(plan->w2_mat, p->alphabet_size);
+        plan->grid_w2 = persistent_grid(ctx, reinterpret_cast<const void *>(fn), plan->w2_smem);
+        const bool few = plan->num_w2 < 2 * plan->grid_w2 * kW2Warps;
+        // A quarter of the batch's time on the device (an SM issues for four warps at once).
+        const double share = 0.25 * cost2 / (4.0 * device_sms(ctx));
         rb2off.assign(N + 1, 0);
         bs2base.assign(N + 1, 0);
+        bool moved = false;
         std::vector<int64_t> bstart(plan->w2b_start.size() + 1, 0);
         size_t bk = 0;
         for (int64_t q = 0; q < plan->num_w2; ++q) {
@@ -1005,8 +1067,30 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
                 if (q == plan->w2b_start[bk]) bstart[bk] = int64_t(w2tasks.size());
             }
             const int32_t k = idx2[q];
-            const int nb = (desc[k].n + kW2BandRows - 1) / kW2BandRows;
-            const bool pipe = nb >= kW2PipeBands || (nb > 1 && few);
+            PairDesc &d = desc[k];
+            bool pipe = plain && few;
+            const double alone = w2_alone(d.m, d.n, d.rows, false);
+            if (!plain && alone > share) {
+                double best = 0.8 * alone;
+                int rows = d.rows;
+                for (int R : {8, 6, 5, 4, 3, 2}) {
+                    if (R > w2_most) continue;
+                    const double c = w2_alone(d.m, d.n, R, true);
+                    if (c < best) {
+                        best = c;
+                        rows = R;
+                        pipe = true;
+                    }
+                    if (c <= share) break;
+                }
+                if (rows != d.rows) {
+                    d.rows = int16_t(rows);
+                    moved = true;
+                    if (plan->traceback) tbytes[k] = w2_trace_bytes(d.m, d.n, rows, plan->local);
+                }
+            }
+            const int nb = w2_bands(d.n, d.rows);
+            pipe = pipe && nb > 1;
             if (pipe) {
                 for (int bb = 0; bb < nb; ++bb) w2tasks.push_back(make_int2(k, bb));
                 bs2base[k] = ns2;
@@ -1016,8 +1100,18 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
             }
             if (nb > 1) {
                 rb2off[k] = rb2tot;
-                rb2tot += (pipe ? 2 : 1) * (int64_t(desc[k].m) + 1);
+                rb2tot += (pipe ? 2 : 1) * (int64_t(d.m) + 1);
             }
+        }
+        if (moved && plan->traceback) {
+            // The pairs' trace sizes changed: lay the traces out again.
+            trace_off = 0;
+            for (int64_t k = 0; k < N; ++k)
+                if (cls[k] != 0) {
+                    desc[k].trace_off = trace_off;
+                    trace_off += tbytes[k];
+                }
+            plan->trace_total = trace_off;
         }
         // Plain form: task ranges per bucket.
         if (!plan->w2b_start.empty()) {
@@ -1030,6 +1124,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     }
     plan->num_w2_tasks = int64_t(w2tasks.size());
     plan->num_w2_states = ns2;
+    plan->num_w2_entries = rb2tot;
     // Per-warp interleaved boundary rows: warp w holds 32 lanes x (max m + 1) int2.
     // (only the one-pair-per-thread strip kernel uses these boundary rows)
     const int64_t warps = (plan->use_warp || p->band_on) ? 0 : (plan->num_slots + 31) / 32;
@@ -1067,7 +1162,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
                          plan->codes_total * 4 + plan->bnd16_total * 8 + plan->num16 * int64_t(sizeof(Slot16)) +
                          plan->seg_slots_total * 16 * 2 + plan->cigar_slots_total * 4 * 2 +
                          plan->seq_h_bytes + plan->seq_v_bytes + rbtot * 8 + nstates * int64_t(sizeof(BandState)) +
-                         plan->num_warp_tasks * 8 + rb2tot * 4 + plan->num_w2 * 12 + plan->num_w2_tasks * 8 +
+                         plan->num_warp_tasks * 8 + rb2tot * 8 + plan->num_w2 * 12 + plan->num_w2_tasks * 8 +
                          ns2 * int64_t(sizeof(BandState));
     if (ctx->budget > 0 && need > ctx->budget)
         return fail(ctx, GBA_EBUDGET, "batch needs %lld bytes of HBM, budget is %lld", (long long)need,
@@ -1076,7 +1171,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     timer.mark("layout");
     if ((rc = upload(ctx, plan->pairs, desc))) return rc;
     if ((rc = upload(ctx, plan->order, idx))) return rc;
-    if ((rc = upload(ctx, plan->warp_scratch, wscr))) return rc;
+    if (scr > 0 && (rc = upload(ctx, plan->warp_scratch, wscr))) return rc;
     GBA_CUDA(ctx, plan->scratch.ensure(size_t(std::max<int64_t>(scr, 1)) * sizeof(int2)));
     if (plan->use_warp && plan->num_slots > 0) {
         if ((rc = upload(ctx, plan->rowbuf_off, rboff))) return rc;
@@ -1089,10 +1184,11 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     }
     if (plan->num_w2 > 0) {
         if ((rc = upload(ctx, plan->tasks_w2, w2tasks))) return rc;
-        if ((rc = upload(ctx, plan->order_w2, idx2))) return rc;
-        if ((rc = upload(ctx, plan->rowbuf_w2_off, rb2off))) return rc;
-        if ((rc = upload(ctx, plan->band_w2_base, bs2base))) return rc;
-        GBA_CUDA(ctx, plan->rowbuf_w2.ensure(size_t(std::max<int64_t>(rb2tot, 1)) * sizeof(uint32_t)));
+        if (plan->traceback && (rc = upload(ctx, plan->order_w2, idx2))) return rc;
+        // (read for pairs of several bands only)
+        if (rb2tot > 0 && (rc = upload(ctx, plan->rowbuf_w2_off, rb2off))) return rc;
+        if (ns2 > 0 && (rc = upload(ctx, plan->band_w2_base, bs2base))) return rc;
+        GBA_CUDA(ctx, plan->rowbuf_w2.ensure(size_t(std::max<int64_t>(rb2tot, 1)) * sizeof(uint64_t)));
         GBA_CUDA(ctx, plan->band_w2.ensure(size_t(std::max<int64_t>(ns2, 1)) * sizeof(BandState)));
         GBA_CUDA(ctx, plan->counter_w2.ensure(std::max<size_t>(16, plan->w2b_start.size() * sizeof(int32_t))));
         GBA_CUDA(ctx, ctx->err_word.ensure(kMaxChunks * sizeof(int32_t)));
@@ -1195,40 +1291,10 @@ WarpLauncher pick_warp(bool a, bool l, bool m, bool t)
     return table[(a ? 8 : 0) | (l ? 4 : 0) | (m ? 2 : 0) | (t ? 1 : 0)];
 }
 
-template <bool A, bool L, bool M, bool T>
-void launch_warp2(const Warp2Args &args, int grid, cudaStream_t s)
+Warp2Fn warp2_fn(bool a, bool l, int mat, bool t)
 {
-    k_dp_warp2<A, L, M, T><<<grid, kBlock, 0, s>>>(args);
-}
-using Warp2Launcher = void (*)(const Warp2Args &, int, cudaStream_t);
-
-Warp2Launcher pick_warp2(bool a, bool l, bool m, bool t)
-{
-    static const Warp2Launcher table[16] = {
-        launch_warp2<false, false, false, false>, launch_warp2<false, false, false, true>,
-        launch_warp2<false, false, true, false>,  launch_warp2<false, false, true, true>,
-        launch_warp2<false, true, false, false>,  launch_warp2<false, true, false, true>,
-        launch_warp2<false, true, true, false>,   launch_warp2<false, true, true, true>,
-        launch_warp2<true, false, false, false>,  launch_warp2<true, false, false, true>,
-        launch_warp2<true, false, true, false>,   launch_warp2<true, false, true, true>,
-        launch_warp2<true, true, false, false>,   launch_warp2<true, true, false, true>,
-        launch_warp2<true, true, true, false>,    launch_warp2<true, true, true, true>};
-    return table[(a ? 8 : 0) | (l ? 4 : 0) | (m ? 2 : 0) | (t ? 1 : 0)];
-}
-
-const void *warp2_fn(bool a, bool l, bool m, bool t)
-{
-#define GBA_W2F(A, L, M, T) (const void *)k_dp_warp2<A, L, M, T>
-    const void *table[16] = {GBA_W2F(false, false, false, false), GBA_W2F(false, false, false, true),
-                             GBA_W2F(false, false, true, false),  GBA_W2F(false, false, true, true),
-                             GBA_W2F(false, true, false, false),  GBA_W2F(false, true, false, true),
-                             GBA_W2F(false, true, true, false),   GBA_W2F(false, true, true, true),
-                             GBA_W2F(true, false, false, false),  GBA_W2F(true, false, false, true),
-                             GBA_W2F(true, false, true, false),   GBA_W2F(true, false, true, true),
-                             GBA_W2F(true, true, false, false),   GBA_W2F(true, true, false, true),
-                             GBA_W2F(true, true, true, false),    GBA_W2F(true, true, true, true)};
-#undef GBA_W2F
-    return table[(a ? 8 : 0) | (l ? 4 : 0) | (m ? 2 : 0) | (t ? 1 : 0)];
+    return a ? (l ? warp2_fn_affine_local(mat, t) : warp2_fn_affine_global(mat, t))
+             : (l ? warp2_fn_linear_local(mat, t) : warp2_fn_linear_global(mat, t));
 }
 
 const void *warp_fn(bool a, bool l, bool m, bool t)
@@ -1379,7 +1445,7 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
         w.seq_v = dseq_v;
         w.pairs = plan->pairs.as<PairDesc>();
         w.tasks = plan->tasks_w2.as<int2>();
-        w.rowbuf = plan->rowbuf_w2.as<uint32_t>();
+        w.rowbuf = plan->rowbuf_w2.as<uint64_t>();
         w.rowbuf_off = plan->rowbuf_w2_off.as<int64_t>();
         w.bands = plan->band_w2.as<BandState>();
         w.band_base = plan->band_w2_base.as<int64_t>();
@@ -1401,11 +1467,14 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
         w.alphabet = plan->matrix ? plan->params.alphabet_size : 0;
         const size_t nb2 = plan->w2b_start.size();
         GBA_CUDA(ctx, cudaMemsetAsync(plan->counter_w2.ptr, 0, sizeof(int32_t) * std::max<size_t>(nb2, 1), ctx->stream));
-        if (plan->num_w2_states > 0)
+        if (plan->num_w2_states > 0) {
             GBA_CUDA(ctx, cudaMemsetAsync(plan->band_w2.ptr, 0, plan->num_w2_states * sizeof(BandState), ctx->stream));
-        const Warp2Launcher wl = pick_warp2(plan->affine, plan->local, plan->matrix, plan->traceback);
+            GBA_CUDA(ctx, cudaMemsetAsync(plan->rowbuf_w2.ptr, 0, plan->num_w2_entries * sizeof(uint64_t), ctx->stream));
+        }
+        const Warp2Fn fn = warp2_fn(plan->affine, plan->local, plan->w2_mat, plan->traceback);
+        auto blocks = [&](int64_t tasks) { return int(std::min<int64_t>(plan->grid_w2, (tasks + kW2Warps - 1) / kW2Warps)); };
         if (nb2 == 0) {
-            wl(w, int(std::min<int64_t>(plan->grid_w2, (plan->num_w2_tasks * 32 + kBlock - 1) / kBlock)), ctx->stream);
+            fn<<<blocks(plan->num_w2_tasks), 32 * kW2Warps, plan->w2_smem, ctx->stream>>>(w);
             ++launches;
         } else {
             // Plain form: one launch per length bucket.
@@ -1414,8 +1483,7 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
                 wb.tasks = w.tasks + plan->w2b_start[b];
                 wb.num_tasks = int32_t(plan->w2b_count[b]);
                 wb.task_counter = w.task_counter + b;
-                wl(wb, int(std::min<int64_t>(plan->grid_w2, (plan->w2b_count[b] * 32 + kBlock - 1) / kBlock)),
-                   ctx->stream);
+                fn<<<blocks(plan->w2b_count[b]), 32 * kW2Warps, plan->w2_smem, ctx->stream>>>(wb);
                 ++launches;
             }
         }
@@ -1613,7 +1681,7 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
             t.num_slots = plan->num_w2;
             t.affine = plan->affine;
             t.local = plan->local;
-            k_traceback_warp<true, kW2Rows><<<warp_blocks(plan->num_w2), kBlock, 0, ctx->stream>>>(t);
+            k_traceback_warp<true, 0><<<warp_blocks(plan->num_w2), kBlock, 0, ctx->stream>>>(t);
             ++launches;
             GBA_CUDA(ctx, cudaGetLastError());
         }

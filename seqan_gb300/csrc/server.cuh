@@ -95,7 +95,12 @@ int64_t request_bytes(const gba_params &p, int64_t m, int64_t n)
     int64_t b = m + n + int64_t(sizeof(PairDesc)) + 128;
     if (p.outputs & GBA_OUT_SEGMENTS) {
         if (p.band_on) b += (m + 1) * band_col_bytes(p.band_upper - p.band_lower + 1) / 32;
-        else b += warp_trace_bytes(int(m), int(n), kWarpRows);
+        else {
+            int64_t t = warp_trace_bytes(int(m), int(n), kWarpRows);
+            for (int R : {2, 3, 4, 5, 6, 8})
+                t = std::max(t, w2_trace_bytes(int(m), int(n), R, p.mode == GBA_LOCAL));
+            b += t;
+        }
         b += (m + n + 4) * 16 * 2;
     }
     if (!p.band_on && n > 32 * kWarpRows) b += 2 * (m + 1) * 8 + ((n + 255) / 256) * int64_t(sizeof(BandState));

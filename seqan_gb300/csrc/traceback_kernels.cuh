@@ -260,12 +260,12 @@ struct WarpCell {
 };
 struct Warp2Cell {
     const uint8_t *T;
-    int m, n;
-    bool affine;
-    __device__ __forceinline__ int operator()(int c, int r) const { return trace_at_warp2(T, m, n, affine, c, r); }
+    int m, rows;
+    bool local, affine;
+    __device__ __forceinline__ int operator()(int c, int r) const { return w2_trace_at(T, m, rows, local, affine, c, r); }
     __device__ __forceinline__ void prefetch(int c, int r) const
     {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(T + trace_off_warp2(m, n, c, r)));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(T + w2_trace_off(m, rows, local, c, r)));
     }
 };
 
@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(128) k_traceback_warp(TraceArgs a)
     const PairDesc d = a.pairs[p];
     const int lane = threadIdx.x & 31;
     if (W2) {
-        Warp2Cell cell{a.trace + d.trace_off, d.m, d.n, a.affine != 0};
+        Warp2Cell cell{a.trace + d.trace_off, d.m, d.rows, a.local != 0, a.affine != 0};
         WarpSteps<Warp2Cell> steps{cell, lane};
         traceback_pair(a, p, cell, steps, lane == 0);
     } else {
