@@ -7,7 +7,15 @@
 
 void launch_banded_chain(const ChainArgs &a, cudaStream_t st)
 {
-    k_banded_chain<<<unsigned((a.num_chains * 32 + 127) / 128), 128, 0, st>>>(a);   // one warp per chain
+    constexpr size_t smem = 4 * chain::kSharedPerWarp;   // one warp per chain, four per block
+    cudaFuncSetAttribute(k_banded_chain, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    int device = 0, sms = 1, per_sm = 1;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_banded_chain, 128, smem);
+    const int64_t resident = int64_t(sms) * (per_sm > 0 ? per_sm : 1), wanted = (a.num_chains + 3) / 4;
+    cudaMemsetAsync(a.next, 0, sizeof(int32_t), st);
+    k_banded_chain<<<unsigned(wanted < resident ? wanted : resident), 128, smem, st>>>(a);
 }
 
 void launch_chain_pack(const chain::ChainDesc *chains, int64_t num_chains, const uint8_t *arena, int32_t max_traces,

@@ -1,7 +1,7 @@
 // chain_host.cuh -- host side of gba_banded_chain (included at the end of engine.cu).
 //
 // A host pass runs every chain's driver in plan mode (grid geometry only) to size its scratch;
-// chains are then processed in chunks whose scratch fits kChainArenaBudget: one thread per chain
+// chains are then processed in chunks whose scratch fits kChainArenaBudget: one warp per chain
 // runs the whole chain (k_banded_chain), the per-chain trace lengths come back, the host lays out
 // the dense output and k_chain_pack copies each chain's first trace there.
 #pragma once
@@ -78,7 +78,6 @@ GBA_API int gba_banded_chain(gba_context *ctx, const gba_chain_params *params, c
         chain::Engine e{};
         e.plan = true;
         e.warp = false;
-        e.lane = 0;
         e.anchor = anchor;
         e.gap = gap;
         e.fe = params->free_ends;
@@ -128,7 +127,14 @@ GBA_API int gba_banded_chain(gba_context *ctx, const gba_chain_params *params, c
         GBA_CUDA(ctx, ctx->bc_desc.ensure(size_t(nc) * sizeof(chain::ChainDesc)));
         GBA_CUDA(ctx, ctx->bc_arena.ensure(size_t(tot) + 16));
         GBA_CUDA(ctx, ctx->bc_out.ensure(size_t(nc) * 16 + 64));
-        GBA_CUDA(ctx, cudaMemcpyAsync(ctx->bc_desc.ptr, desc.data() + c0, size_t(nc) * sizeof(chain::ChainDesc),
+        // Longest chains first: a warp runs one chain from end to end, so a long one taken last would
+        // leave the device to itself.
+        for (int64_t k = c0; k < c1; ++k) desc[k].id = int32_t(k - c0);
+        std::vector<chain::ChainDesc> order(desc.begin() + c0, desc.begin() + c1);
+        std::stable_sort(order.begin(), order.end(), [](const chain::ChainDesc &x, const chain::ChainDesc &y) {
+            return x.plan.cells > y.plan.cells;
+        });
+        GBA_CUDA(ctx, cudaMemcpyAsync(ctx->bc_desc.ptr, order.data(), size_t(nc) * sizeof(chain::ChainDesc),
                                       cudaMemcpyHostToDevice, st));
         int32_t *o = ctx->bc_out.as<int32_t>();
         ChainArgs a{};
@@ -148,6 +154,7 @@ GBA_API int gba_banded_chain(gba_context *ctx, const gba_chain_params *params, c
         a.status = o + nc;
         a.n_traces = o + 2 * nc;
         a.seg_count = o + 3 * nc;
+        a.next = o + 4 * nc;
         GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));
         launch_banded_chain(a, st);
         GBA_CUDA(ctx, cudaGetLastError());

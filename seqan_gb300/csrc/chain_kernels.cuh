@@ -1,13 +1,17 @@
 // chain_kernels.cuh -- banded chain alignment (bandedChainAlignment over a seed chain,
-// seeds/banded_chain_alignment*.h), one chain per thread.
+// seeds/banded_chain_alignment*.h), one chain per warp.
 //
 // A chain is a sequence of grids -- the rectangle before the first anchor, then per anchor a band
 // around it and the rectangle to the next anchor, then the rectangle to the matrix end -- each a
 // DP whose first row and column come from cells the previous grid's traceback picked.  The grids
-// of one chain depend on each other; chains are independent, so a batch runs one chain per thread
-// with the chain's scratch (trace matrix of the current grid, two score columns, the four init
-// vectors, the init-cell set, the positions of the maximum and the trace sets) in its own slice of
-// an HBM arena.  The same code runs on the host in plan mode: the grids' geometry depends only on
+// of one chain depend on each other; chains are independent, so a batch runs one chain per warp, with
+// the driver's state, the current grid's trace and its columns in shared memory and the chain's other
+// scratch (four init vectors, the init-cell set, the positions of the maximum and the trace sets;
+// the trace and columns of grids too large for shared memory) in its own slice of an HBM arena.
+// Bound by the latency of a warp's own instructions: 16 warps fit an SM beside their shared memory,
+// and a grid's diagonals, tracebacks and glue follow one another.  Measured on 10,000 chains of
+// 1-3 kbp (band extension 15), whole call: 190 -> 45 ms; of a chain's 131M cycles the fill took 112M
+// before, with 28 warps on an SM, and takes 10M of 15M now with 16.  The same code runs on the host in plan mode: the grids' geometry depends only on
 // the seeds, the band extension and the sequence lengths, so a host pass sizes every chain's
 // slice before the kernel runs.
 //
@@ -68,14 +72,20 @@ struct Plan {
 };
 
 // One column of a grid as the reference's loop visits it: rows r0..r1 (r1 = r0 for a single
-// cell), its column type and location, the trace navigator's position at its first cell and the
-// lane leap its cells see.
-struct ColDesc {
-    int r0, r1;
-    int64_t pos0;
-    int leap;
-    int hcol, vrow0;   // storage column and storage row of the first cell (a column never wraps)
-    int8_t type, loc, single, present;
+// cell) and the trace navigator's position at its first cell, what its cells are, the rows the scout
+// stores and tracks, and its candidate for the maximum.
+enum : int { CD_INITIAL = 1, CD_PRESET = 2, CD_LOWER = 4, CD_FINAL = 8 };
+struct alignas(16) ColDesc {
+    int r0, r1, pos0;
+    int kind;          // CD_INITIAL: given by the first column's entries from `entry` on; CD_PRESET: the
+                       // first cell given by the first row's; CD_LOWER: the last cell without the
+                       // horizontal direction; CD_FINAL: the last column
+    int rowStore;      // row stored for the next grid's first row, or -1
+    int rowCol;        // rows from here on stored for its first column
+    int rowTrack;      // rows from here on tracked
+    int entry;         // index of the given cells / of this column in the stored row
+    int candS, candP;  // last cell's score and position when it is tracked (position -1: not)
+    int pad[2];
 };
 
 // One chain's scratch slices (device or host memory) and its inputs.
@@ -91,22 +101,39 @@ struct Work {
     Seg *lseg;      // local traces: slot q at lseg + q * lseg_cap, reference order
     int *llen;      // [traces]
     int *erase;     // [traces]
-    // warp-cooperative fill: per-column descriptors, three rolling anti-diagonals of (S, E, F)
-    // indexed by column, candidate cells for the maximum (last cell per column, the final column)
+    // warp-cooperative fill: per-column descriptors and the final column's candidates for the maximum
     ColDesc *cols;
-    int *aS, *aE, *aF;       // [3 * col_cap]
-    int *ccS, *ccP, *ccF;    // [col_cap]
-    int *fcS, *fcP, *fcF;    // [col_rows]
+    int *fcS, *fcP;          // [col_rows]; position -1: not a candidate
+    // the warp's shared memory: a grid whose trace (descriptors) fits there keeps them there
+    uint8_t *sharedT;
+    ColDesc *sharedCols;
+    uint8_t *arenaT;
+    ColDesc *arenaCols;
 };
+
+// Shared memory of one warp.  The bands and rectangles of a band extension of 15 take 3-6 KB of trace
+// and 30-90 columns; four blocks of four warps then share an SM.
+constexpr int kSharedTrace = 7680;
+constexpr int kSharedCols = 112;
 
 
 struct ChainDesc {
     int64_t h_off, v_off, seed_off;   // into the batch's codes and seeds (4 int32 per seed)
     int32_t m, n, n_seeds;
-    int32_t pad;
+    int32_t id;                       // its place in the batch (the chains run longest first)
     int64_t arena_off;                // byte offset of the chain's scratch
     Plan plan;
 };
+
+// The driver calls the steps of a grid from seven places; with a copy of each in every place the
+// kernel ran out of instruction cache (ncu: 8.9 of 16 stall cycles an instruction).
+#if defined(__CUDACC__)
+#define GBA_CHAIN_STEP __noinline__
+#define GBA_CHAIN_INLINE __forceinline__
+#else
+#define GBA_CHAIN_STEP
+#define GBA_CHAIN_INLINE inline
+#endif
 
 template <typename T> __host__ __device__ inline T cmin(T a, T b) { return a < b ? a : b; }
 template <typename T> __host__ __device__ inline T cmax(T a, T b) { return a > b ? a : b; }
@@ -124,7 +151,6 @@ struct Engine {
     // ---- configuration ----
     bool plan;                  // plan mode: geometry only
     bool warp;                  // one warp per chain: grids filled by anti-diagonals across the lanes
-    int lane;                   // this thread's lane (0 on the host)
     Scheme anchor, gap;
     int fe, affine, k;
     int max_traces;
@@ -159,9 +185,12 @@ struct Engine {
     Cell bestCell;
 
     __host__ __device__ void fail(int code) { if (!err) err = code; }
+#ifdef __CUDA_ARCH__
+    static __device__ __forceinline__ int lane_id() { return int(threadIdx.x & 31); }
+#endif
 
     // =========================== init-cell set ===========================
-    __host__ __device__ bool set_insert(int i1, int i2, Cell c)
+    GBA_CHAIN_STEP __host__ __device__ bool set_insert(int i1, int i2, Cell c)
     {
         if (plan) return true;
         int lo = 0, hi = nset;
@@ -182,7 +211,7 @@ struct Engine {
     }
 
     // _reinitScoutState
-    __host__ __device__ void reinit(int64_t oh, int64_t ov, int64_t ch, int64_t cv, int64_t nh, int64_t nv)
+    GBA_CHAIN_STEP __host__ __device__ void reinit(int64_t oh, int64_t ov, int64_t ch, int64_t cv, int64_t nh, int64_t nv)
     {
         if (err) return;
         const int64_t want[4] = {ch, cv, nh, nv};
@@ -198,7 +227,7 @@ struct Engine {
             }
 #ifdef __CUDA_ARCH__
             if (warp) {
-                for (int i = lane; i < n4[q]; i += 32) w.v4[q][i] = Cell{INF, INF, INF};
+                for (int i = lane_id(); i < n4[q]; i += 32) w.v4[q][i] = Cell{INF, INF, INF};
                 continue;
             }
 #endif
@@ -226,7 +255,7 @@ struct Engine {
     __host__ __device__ Seg *gslot(int q) { return w.gseg + int64_t(q) * pl->gseg_cap; }
 
     // _recordSegment into local trace q (q < 0: discarded)
-    __host__ __device__ void record(int q, int64_t hp, int64_t vp, int64_t len, int tv)
+    GBA_CHAIN_STEP __host__ __device__ void record(int q, int64_t hp, int64_t vp, int64_t len, int tv)
     {
         if (len == 0 || q < 0) return;
         int type;
@@ -296,7 +325,7 @@ struct Engine {
     }
 
     // _adaptLocalTracesToGlobalGrid + _glueTracebacks (check_empty: skip an empty local set)
-    __host__ __device__ void glue_local(int64_t gbh, int64_t gbv, bool check_empty)
+    GBA_CHAIN_STEP __host__ __device__ void glue_local(int64_t gbh, int64_t gbv, bool check_empty)
     {
         if (plan || err) return;
         for (int i = 0; i < nl; ++i) {
@@ -471,7 +500,7 @@ struct Engine {
     }
 
     // one cell: navigator step, value, trace byte, tracking
-    __host__ __device__ void cell(int coltype, int loc, int cellk, int col, int row)
+    GBA_CHAIN_STEP __host__ __device__ void cell(int coltype, int loc, int cellk, int col, int row)
     {
         if (err) return;
         nav_move(coltype, loc, cellk);
@@ -619,7 +648,7 @@ struct Engine {
         return tv;
     }
 
-    __host__ __device__ void track_col(int col, int coltype, int loc, int r0, int r1)
+    GBA_CHAIN_STEP __host__ __device__ void track_col(int col, int coltype, int loc, int r0, int r1)
     {
         new_col(col);
         dS = INF; vS = INF; vF = INF;
@@ -740,22 +769,25 @@ struct Engine {
 
     // ---------------- traceback over the band storage ----------------
     struct Walk {
-        int64_t pos, cc, cr, ec, er, bp1, bp2;
+        int pos, cc, cr, ec, er, bp1, bp2;   // (positions and grid sizes are below 2^31)
         int tv, last;
-        int64_t frag;
+        int frag;
+        int stride, cells;                   // L and L * Hlen
         bool band, bad;
     };
 
     __host__ __device__ void coord_init(Walk &wk, int64_t cc, int64_t cr, int64_t ec, int64_t er) const
     {
-        wk.cc = cc; wk.cr = cr; wk.ec = ec; wk.er = er; wk.bp1 = 0; wk.bp2 = 0; wk.band = false;
+        wk.stride = int(L);
+        wk.cells = int(L * Hlen);
+        wk.cc = int(cc); wk.cr = int(cr); wk.ec = int(ec); wk.er = int(er); wk.bp1 = 0; wk.bp2 = 0; wk.band = false;
         if (banded) {
             if (lower >= 0) wk.cc += lower;
             if (wk.cc > upper) wk.cr += wk.cc - upper;
             if (wk.ec > upper) wk.er += wk.ec - upper;
-            wk.bp1 = cmin<int64_t>(gm, cmax<int64_t>(0, upper));
-            wk.bp2 = cmin<int64_t>(gm, cmax<int64_t>(0, int64_t(gn) + lower));
-            const int64_t b = cmin(wk.bp1, wk.bp2);
+            wk.bp1 = int(cmin<int64_t>(gm, cmax<int64_t>(0, upper)));
+            wk.bp2 = int(cmin<int64_t>(gm, cmax<int64_t>(0, int64_t(gn) + lower)));
+            const int b = cmin(wk.bp1, wk.bp2);
             if (wk.cc < b) wk.cr -= b - wk.cc;
             wk.band = true;
         }
@@ -776,14 +808,14 @@ struct Engine {
         return T_NONE;
     }
 
-    __host__ __device__ void w_step(Walk &wk, int64_t d) const
+    __host__ __device__ GBA_CHAIN_INLINE void w_step(Walk &wk, int d) const
     {
         if (d <= 0) { wk.bad = true; wk.tv = T_NONE; return; }   // a one-row band: the walk would not move
         wk.pos -= d;
-        if (wk.pos < 0 || wk.pos >= L * Hlen) { wk.bad = true; wk.tv = T_NONE; return; }
+        if (wk.pos < 0 || wk.pos >= wk.cells) { wk.bad = true; wk.tv = T_NONE; return; }
         wk.tv = w.T[wk.pos];
     }
-    __host__ __device__ void w_switch(Walk &wk, int q, int bit)
+    __host__ __device__ GBA_CHAIN_INLINE void w_switch(Walk &wk, int q, int bit)
     {
         if (!(wk.last & bit)) {
             record(q, wk.cc, wk.cr, wk.frag, wk.last);
@@ -792,12 +824,12 @@ struct Engine {
         }
     }
     // _doTraceback with GapsLeft
-    __host__ __device__ void do_trace(Walk &wk, int q)
+    __host__ __device__ GBA_CHAIN_INLINE void do_trace(Walk &wk, int q)
     {
         const int tv = wk.tv;
         if (tv & T_DIAG) {
             w_switch(wk, q, T_DIAG);
-            w_step(wk, in_band(wk) ? L : L + 1);
+            w_step(wk, in_band(wk) ? wk.stride : wk.stride + 1);
             --wk.cc; --wk.cr; ++wk.frag;
         } else if ((tv & T_MFV) && (tv & T_V)) {
             w_switch(wk, q, T_V);
@@ -816,14 +848,14 @@ struct Engine {
             w_switch(wk, q, T_H);
             if (affine)
                 while ((!(wk.tv & T_HO) || (wk.tv & T_H)) && wk.cc != 1 && !wk.bad) {
-                    w_step(wk, in_band(wk) ? L - 1 : L);
+                    w_step(wk, in_band(wk) ? wk.stride - 1 : wk.stride);
                     --wk.cc; ++wk.frag;
                 }
-            w_step(wk, in_band(wk) ? L - 1 : L);
+            w_step(wk, in_band(wk) ? wk.stride - 1 : wk.stride);
             --wk.cc; ++wk.frag;
         } else if ((tv & T_MFH) && (tv & T_HO)) {
             w_switch(wk, q, T_H);
-            w_step(wk, in_band(wk) ? L - 1 : L);
+            w_step(wk, in_band(wk) ? wk.stride - 1 : wk.stride);
             --wk.cc; ++wk.frag;
         } else {
             wk.bad = true;   // a trace value the reference asserts on: its walk never ends
@@ -837,7 +869,7 @@ struct Engine {
     }
 
     // the generic _computeTraceback from position *p (no head / tail for the chain profile)
-    __host__ __device__ void generic_trace(int q, int64_t &p)
+    GBA_CHAIN_STEP __host__ __device__ void generic_trace(int q, int &p)
     {
         Walk wk;
         wk.pos = p; wk.bad = false; wk.frag = 0;
@@ -859,17 +891,17 @@ struct Engine {
     }
 
     // the chain's traceback from one position of the maximum
-    __host__ __device__ void chain_trace_one(int64_t maxpos)
+    GBA_CHAIN_STEP __host__ __device__ void chain_trace_one(int64_t maxpos)
     {
         const int q = new_local();
         if (q < 0) return;
         Walk wk;
-        wk.pos = maxpos; wk.bad = false; wk.frag = 0;
+        wk.pos = int(maxpos); wk.bad = false; wk.frag = 0;
         wk.tv = w.T[maxpos];
         wk.last = initial_dir(wk.tv, prefer_end());
         coord_init(wk, maxpos / L, maxpos % L, hNext, vNext);
         if (kind == KIND_FINAL) {
-            int64_t p = maxpos;
+            int p = int(maxpos);
             if (wk.cr != gn) record(q, gm, wk.cr, gn - wk.cr, T_V);
             if (wk.cc != gm) record(q, wk.cc, wk.cr, gm - wk.cc, T_H);
             generic_trace(q, p);
@@ -906,12 +938,12 @@ struct Engine {
     }
 
     // the standard traceback of a GlobalAlignment_ grid (head and tail, no start-cell correction)
-    __host__ __device__ void global_trace()
+    GBA_CHAIN_STEP __host__ __device__ void global_trace()
     {
         const int q = new_local();
         if (q < 0) return;
         Walk wk;
-        wk.pos = bestPos; wk.bad = false; wk.frag = 0;
+        wk.pos = int(bestPos); wk.bad = false; wk.frag = 0;
         wk.tv = w.T[bestPos];
         wk.last = initial_dir(wk.tv, prefer_end());
         coord_init(wk, bestPos / L, bestPos % L, 0, 0);
@@ -925,7 +957,7 @@ struct Engine {
     }
 
     // _computeAlignment of one grid; local traces go to the local set (appended)
-    __host__ __device__ int run_grid(const Scheme *s, int kd, bool bd, int lw, int up, const uint8_t *ph, int64_t pm,
+    GBA_CHAIN_STEP __host__ __device__ int run_grid(const Scheme *s, int kd, bool bd, int lw, int up, const uint8_t *ph, int64_t pm,
                                      const uint8_t *pv, int64_t pn)
     {
         if (err) return INT_MIN;
@@ -974,9 +1006,15 @@ struct Engine {
             return 0;
         }
         if (L * Hlen > pl->trace_bytes || pn + 1 > pl->col_rows) { fail(ST_CAPACITY); return INT_MIN; }
-        if (!warp || kd == KIND_GLOBAL) {
-            for (int64_t q = 0; q < L * Hlen; ++q) w.T[q] = 0;
-        }
+#ifdef __CUDA_ARCH__
+        w.T = L * Hlen <= kSharedTrace ? w.sharedT : w.arenaT;
+        w.cols = pm + 1 <= kSharedCols ? w.sharedCols : w.arenaCols;
+        __syncwarp();
+        for (int64_t q = lane_id(); q < (L * Hlen + 15) / 16; q += 32) reinterpret_cast<uint4 *>(w.T)[q] = make_uint4(0, 0, 0, 0);
+        __syncwarp();
+#else
+        for (int64_t q = 0; q < L * Hlen; ++q) w.T[q] = 0;
+#endif
         lo0 = lo1 = INT_MAX;
         hi0 = hi1 = -1;
         maxS = INF;
@@ -998,53 +1036,97 @@ struct Engine {
     }
 
     // ---------------- warp-cooperative fill ----------------
-    // The cells of one anti-diagonal (c + r = d) depend only on the two before it, so the lanes of a
-    // warp take the cells of a diagonal together.  Every cell gets the inputs the column-major loop
-    // gives it -- the horizontal and diagonal neighbours from the previous column's computed rows,
-    // the cell above as cacheVert (none for a column's first cell), the diagonal preset of middle /
-    // bottom columns -- so values, trace bytes and init-vector stores are the loop's.  The candidates
-    // for the maximum are kept per column and scanned afterwards in column-major order, which gives
-    // the scout's list of positions in the loop's order.
-
-    static __host__ __device__ int64_t floor2(int64_t a) { return a >= 0 ? a / 2 : -((-a + 1) / 2); }
-
-    __host__ __device__ void desc_col(int col, int coltype, int loc, int r0, int r1, bool single, int64_t &p,
-                                      int64_t &lp)
+    // The lanes take the columns of a grid in turn (lane l: columns l, l + 32, ...) and step through
+    // the anti-diagonals d = c + r together, so a cell's horizontal neighbour is what the lane to the
+    // left computed one step before and its diagonal neighbour what that lane handed over the step
+    // before that; the cell above is the lane's own last one.  All of it stays in registers (three
+    // rolling diagonals in global scratch took about 10,000 cycles a diagonal with 28 warps on the SM;
+    // a step takes about 700 with 16).  A lane goes on to its next column when a column ends; where columns are
+    // so tall that the next one would already have begun, the columns are swept in blocks of 32
+    // instead and the last lane hands its column to the next block through scratch.  Every cell gets
+    // the inputs the column-major loop gives it -- the neighbours from the previous column's computed
+    // rows, the cell above as cacheVert (none for a column's first cell), the diagonal preset of
+    // middle / bottom columns -- so values, trace bytes and init-vector stores are the loop's.  The
+    // candidates for the maximum are kept per column and collected afterwards in column-major order,
+    // which gives the scout's list of positions in the loop's order.
+    // Measured (10,000 chains of 1-3 kbp): whole call BEFORE -> AFTER ms.
+#ifdef __CUDA_ARCH__
+    // n columns from col on, the q-th with rows r0 + q * dr0 .. r1 + q * dr1 (single: one cell);
+    // p, lp: the navigator's position and leap after the previous column, advanced past the run.
+    // The lanes write the run's descriptors in closed form.
+    GBA_CHAIN_STEP __device__ void columns(int col, int n, int type, int loc, int r0, int r1, int dr0, int dr1, bool single,
+                            int64_t &p, int64_t &lp)
     {
-        if (col < 0 || col > gm || col >= pl->col_cap) { fail(ST_UNDEFINED); return; }
-        if (!single && r1 <= r0) { fail(ST_UNDEFINED); return; }   // the reference's track needs two cells
-        if (coltype != COL_INITIAL) {
-            if (banded && loc == LOC_TOP) { lp -= 1; p += lp; }
-            else p += lp;
+        if (n <= 0) return;
+        if (col < 0 || col + n - 1 > gm || col + n > pl->col_cap) { fail(ST_UNDEFINED); return; }
+        const bool initial = type == COL_INITIAL;
+        const int hN = int(hNext), vN = int(vNext);
+        const bool top = banded && loc == LOC_TOP && !initial, bottom = banded && loc == LOC_BOTTOM && !initial;
+        const int64_t h0 = single ? 0 : r1 - r0, dh = single ? 0 : dr1 - dr0;
+        // the q-th column's position: the leaps so far and the rows of the columns before it
+        auto first = [&](int64_t q) {
+            const int64_t leaps = initial ? 0 : (q + 1) * lp + (top ? -(q + 1) * (q + 2) / 2 : (bottom ? q * (q + 1) / 2 : 0));
+            return p + leaps + q * h0 + dh * (q * (q - 1) / 2);
+        };
+        for (int q = lane_id(); q < n; q += 32) {
+            const int64_t pos0 = first(q), rows = h0 + q * dh;
+            if ((!single && rows <= 0) || pos0 < 0 || pos0 + rows >= L * Hlen) {   // the reference's track needs two cells
+                fail(ST_UNDEFINED);
+                continue;
+            }
+            ColDesc d;
+            d.r0 = r0 + q * dr0;
+            d.r1 = d.r0 + int(rows);
+            d.pos0 = int(pos0);
+            d.kind = (initial ? CD_INITIAL : (loc == LOC_TOP || loc == LOC_FULL ? CD_PRESET : 0)) |
+                     (loc == LOC_TOP || loc == LOC_MIDDLE ? CD_LOWER : 0) | (type == COL_FINAL ? CD_FINAL : 0);
+            d.rowStore = -1;
+            d.rowCol = d.rowTrack = INT_MAX;
+            d.candS = INF;
+            d.candP = -1;
+            d.pad[0] = d.pad[1] = 0;
+            const int hcol = int(uint32_t(pos0) / uint32_t(L)), vrow0 = int(pos0) - hcol * int(L);   // storage cell
+            const int clp = int(top ? lp - (q + 1) : (bottom ? lp + q : lp));                        // leap
+            if (!single && vrow0 + rows >= L) fail(ST_UNDEFINED);
+            // the given cells: the first column's entries vrow0 - leap + 1 .., the first row's entry hcol
+            d.entry = initial ? vrow0 - (clp - 1) : hcol;
+            if (initial ? (d.entry < 0 || d.entry + rows >= n4[1]) : ((d.kind & CD_PRESET) && hcol >= n4[0])) fail(ST_UNDEFINED);
+            // the chain's tracking options
+            if (hcol >= hN) {
+                const int row = d.r0 + vN - vrow0;          // the row of storage row vN
+                int at = row - (loc == LOC_BOTTOM ? clp : 0);
+                // a bottom column's last cell sees a leap one larger
+                if (loc == LOC_BOTTOM && !initial && rows > 0) at = at - 1 == d.r1 ? d.r1 : (at == d.r1 ? -1 : at);
+                if (at >= d.r0 && at <= d.r1) {
+                    d.rowStore = at;
+                    if (hcol - hN >= n4[2] || (initial && hcol != hN)) fail(ST_UNDEFINED);
+                }
+                if (hcol == hN && row <= d.r1) {
+                    d.rowCol = row;
+                    if (d.r1 - row >= n4[3]) fail(ST_UNDEFINED);
+                }
+                const bool finalM = kind == KIND_FINAL;
+                if (type == COL_FINAL && (!finalM || (fe & FREE_RIGHT))) d.rowTrack = loc != LOC_FULL ? d.r0 : cmin(row, d.r1);
+                else if (rows > 0 && (type == COL_FINAL || !finalM || (fe & FREE_BOTTOM))) d.rowTrack = d.r1;
+                // (a single cell of the final column is its first one: tracked as a row, never as the last)
+            }
+            w.cols[col + q] = d;
         }
-        ColDesc &d = w.cols[col];
-        d.r0 = r0;
-        d.r1 = single ? r0 : r1;
-        d.pos0 = p;
-        d.leap = int(lp);
-        d.hcol = int(p / L);
-        d.vrow0 = int(p % L);
-        if (!single && d.vrow0 + (r1 - r0) >= L) { fail(ST_UNDEFINED); return; }
-        d.type = int8_t(coltype);
-        d.loc = int8_t(loc);
-        d.single = single;
-        d.present = 1;
-        if (!single) {
-            p += r1 - r0;
-            if (banded && loc == LOC_BOTTOM && coltype != COL_INITIAL) lp += 1;
-        }
+        __syncwarp();
+        p = first(n - 1) + h0 + (n - 1) * dh;
+        lp = top ? lp - n : (bottom && !single ? lp + n : lp);
     }
 
     // the columns of run_banded / run_unbanded, with the navigator's positions
-    __host__ __device__ void describe(int &cfirst, int &clast)
+    __device__ void describe(int &cfirst, int &clast)
     {
         int64_t p = pos, lp = leap;
         cfirst = 0;
         clast = gm;
         if (!banded) {
-            desc_col(0, COL_INITIAL, LOC_FULL, 0, gn, false, p, lp);
-            for (int c = 1; c < gm; ++c) desc_col(c, COL_INNER, LOC_FULL, 0, gn, false, p, lp);
-            desc_col(gm, COL_FINAL, LOC_FULL, 0, gn, false, p, lp);
+            columns(0, 1, COL_INITIAL, LOC_FULL, 0, gn, 0, 0, false, p, lp);
+            columns(1, gm - 1, COL_INNER, LOC_FULL, 0, gn, 0, 0, false, p, lp);
+            columns(gm, 1, COL_FINAL, LOC_FULL, 0, gn, 0, 0, false, p, lp);
             return;
         }
         const int mm = gm, nn = gn, lw = lower, up = upper;
@@ -1056,217 +1138,265 @@ struct Engine {
         if (hb == mm - 1) {
             const int col = cmax(0, cmin(mm, lw));
             cfirst = clast = col;
-            desc_col(col, COL_INITIAL, LOC_TOP, 0, 0, true, p, lp);
+            columns(col, 1, COL_INITIAL, LOC_TOP, 0, 0, 0, 0, true, p, lp);
             return;
         }
         if (hBot == 0) {
             const int row = cmin(nn, -up);
             cfirst = clast = 0;
-            desc_col(0, COL_INITIAL, LOC_BOTTOM, row, row, true, p, lp);
+            columns(0, 1, COL_INITIAL, LOC_BOTTOM, row, row, 0, 0, true, p, lp);
             return;
         }
         if (up < 0) {
             ++vb;
-            desc_col(0, COL_INITIAL, lw > -nn ? LOC_MIDDLE : LOC_BOTTOM, vb, ve, false, p, lp);
+            columns(0, 1, COL_INITIAL, lw > -nn ? LOC_MIDDLE : LOC_BOTTOM, vb, ve, 0, 0, false, p, lp);
         } else if (lw >= 0) {
             cfirst = hb;
-            desc_col(hb, COL_INITIAL, LOC_TOP, 0, 0, true, p, lp);
+            columns(hb, 1, COL_INITIAL, LOC_TOP, 0, 0, 0, 0, true, p, lp);
         } else {
-            desc_col(0, COL_INITIAL, lw <= -nn ? LOC_FULL : LOC_TOP, vb, ve, false, p, lp);
+            columns(0, 1, COL_INITIAL, lw <= -nn ? LOC_FULL : LOC_TOP, vb, ve, 0, 0, false, p, lp);
         }
         int hIt = hb;
-        for (; hIt != hTop && !err; ++hIt) { ++ve; desc_col(hIt + 1, COL_INNER, LOC_TOP, vb, ve, false, p, lp); }
-        if (up > nn + lw) {
-            for (; hIt != hMid && !err; ++hIt) desc_col(hIt + 1, COL_INNER, LOC_FULL, vb, ve, false, p, lp);
-        } else {
-            for (; hIt != hMid && !err; ++hIt) {
-                ++vb; ++ve;
-                desc_col(hIt + 1, COL_INNER, LOC_MIDDLE, vb, ve, false, p, lp);
-            }
-        }
-        for (; hIt != hBot && !err; ++hIt) { ++vb; desc_col(hIt + 1, COL_INNER, LOC_BOTTOM, vb, ve, false, p, lp); }
+        auto run = [&](int to, int loc, int db, int de) {
+            const int n = cmax(0, to - hIt);
+            columns(hIt + 1, n, COL_INNER, loc, vb + db, ve + de, db, de, false, p, lp);
+            vb += n * db;
+            ve += n * de;
+            hIt += n;
+        };
+        run(hTop, LOC_TOP, 0, 1);
+        if (up > nn + lw) run(hMid, LOC_FULL, 0, 0);
+        else run(hMid, LOC_MIDDLE, 1, 1);
+        run(hBot, LOC_BOTTOM, 1, 0);
         clast = hIt;
         if (hIt < mm - 1) {
             clast = hIt + 1;
-            desc_col(hIt + 1, COL_INNER, LOC_BOTTOM, vb + 1, vb + 1, true, p, lp);
+            columns(hIt + 1, 1, COL_INNER, LOC_BOTTOM, vb + 1, vb + 1, 0, 0, true, p, lp);
         } else if (hIt == mm - 1) {
             clast = mm;
-            if (up == mm - nn) desc_col(mm, COL_FINAL, LOC_BOTTOM, vb + 1, vb + 1, true, p, lp);
+            if (up == mm - nn) columns(mm, 1, COL_FINAL, LOC_BOTTOM, vb + 1, vb + 1, 0, 0, true, p, lp);
             else if (up >= mm) {
-                if (lw + nn > mm) { ++ve; desc_col(mm, COL_FINAL, LOC_TOP, vb, ve, false, p, lp); }
-                else if (lw + nn + 1 > mm) { ++ve; desc_col(mm, COL_FINAL, LOC_TOP, vb, ve, false, p, lp); }
-                else desc_col(mm, COL_FINAL, LOC_FULL, vb, ve, false, p, lp);
+                if (lw + nn + 1 > mm) { ++ve; columns(mm, 1, COL_FINAL, LOC_TOP, vb, ve, 0, 0, false, p, lp); }
+                else columns(mm, 1, COL_FINAL, LOC_FULL, vb, ve, 0, 0, false, p, lp);
             } else {
                 ++vb;
-                if (lw + nn <= mm) {
-                    if (lw + nn == mm) { ++ve; desc_col(mm, COL_FINAL, LOC_MIDDLE, vb, ve, false, p, lp); }
-                    else desc_col(mm, COL_FINAL, LOC_BOTTOM, vb, ve, false, p, lp);
+                if (lw + nn < mm) {
+                    columns(mm, 1, COL_FINAL, LOC_BOTTOM, vb, ve, 0, 0, false, p, lp);
                 } else {
                     ++ve;
-                    desc_col(mm, COL_FINAL, LOC_MIDDLE, vb, ve, false, p, lp);
+                    columns(mm, 1, COL_FINAL, LOC_MIDDLE, vb, ve, 0, 0, false, p, lp);
                 }
             }
         }
     }
 
-    // the cells of anti-diagonal d that lane l takes; k3 / k1 / k2: the rolling slots of d, d - 1, d - 2
-    __host__ __device__ void fill_diag(int d, int l, int cfirst, int clast, int k3, int k1, int k2)
+    // Columns cbeg .. cend, anti-diagonals dlo .. dhi.  wrap: a lane goes on to its next column; else
+    // cend - cbeg < 32 and the column before cbeg comes from scratch.
+    template <bool AFFINE>
+    GBA_CHAIN_STEP __device__ void sweep(int cfirst, int cbeg, int cend, bool wrap, int dlo, int dhi)
     {
-        const int cap = pl->col_cap, gnn = gn;
-        const int hN = int(hNext), vN = int(vNext);
-        const bool finalM = kind == KIND_FINAL;
-        const bool freeB = (fe & FREE_BOTTOM) != 0, freeR = (fe & FREE_RIGHT) != 0;
-        const ColDesc *cols = w.cols;
-        int *aS = w.aS, *aE = w.aE, *aF = w.aF;
-        int clo = cmax(cfirst, d - gnn), chi = cmin(clast, d);
-        if (banded) {
-            clo = cmax(clo, int(-floor2(-(int64_t(d) + lower))));
-            chi = cmin(chi, int(floor2(int64_t(d) + upper)));
-        }
-        for (int c = clo + l; c <= chi; c += 32) {
-            const int r = d - c;
-            const ColDesc cd = cols[c];
-            if (!cd.present || r < cd.r0 || r > cd.r1) continue;
-            const int cellk = (r == cd.r0) ? CELL_FIRST : (r == cd.r1 ? CELL_LAST : CELL_INNER);
-            const int dr = r - cd.r0;
-            const int p = int(cd.pos0) + dr;
-            const int lp = cd.leap + ((cellk == CELL_LAST && cd.loc == LOC_BOTTOM && cd.type != COL_INITIAL) ? 1 : 0);
-            // the previous column's computed rows
-            bool hv = false, dv = false;
+        ColDesc *const cols = w.cols;
+        uint8_t *const T = w.T;
+        const int stored = int(hNext);
+        const int ext = sc->ext, open = sc->open, match = sc->match, mismatch = sc->mismatch;
+        const int lane = lane_id(), left = (lane + 31) & 31;
+        const bool carryIn = !wrap && lane == 0 && cbeg > cfirst, carryOut = !wrap && lane == 31;
+        const uint8_t *const pv = gv, *const ph = gh;
+        Cell *const vTop = w.v4[0], *const vLeft = w.v4[1], *const outRow = w.v4[2], *const outCol = w.v4[3];
+        int *const cS = w.cS0, *const cE = w.cE0, *const fcS = w.fcS, *const fcP = w.fcP;
+        int c = cbeg + lane;
+        // this lane's column: rows r0 .. r0 + h; the previous column's are the po-th before .. prh-th after r0
+        int r0 = 0, h = 0, kind_ = 0, rowStore = -1, rowCol = INT_MAX, rowTrack = INT_MAX, entry = 0;
+        int po = INT_MIN, hc = 0, vc = 0, vcNext = 0, rowAny = INT_MAX;
+        unsigned prh = 0;
+        uint8_t *Tc = T;
+        const uint8_t *vr = pv;                // residue of row r0
+        bool initial = false, preset = false, lower = false;
+        Cell given{INF, INF, INF}, givenNext{INF, INF, INF};
+        auto enter = [&]() {
+            const int4 a = *reinterpret_cast<const int4 *>(&cols[c].r0);
+            const int4 b = *reinterpret_cast<const int4 *>(&cols[c].rowStore);
+            r0 = a.x;
+            h = a.y - a.x;
+            Tc = T + a.z;
+            kind_ = a.w;
+            rowStore = b.x;
+            rowCol = b.y;
+            rowTrack = b.z;
+            entry = b.w;
+            rowAny = cmin(rowCol, rowTrack);
+            if (rowStore >= 0) rowAny = cmin(rowAny, rowStore);
+            initial = (kind_ & CD_INITIAL) != 0;
+            preset = (kind_ & CD_PRESET) != 0;
+            lower = (kind_ & CD_LOWER) != 0;
+            vr = pv + r0 - 1;
             if (c > cfirst) {
-                const ColDesc &pc = cols[c - 1];
-                hv = pc.present && r >= pc.r0 && r <= pc.r1;
-                dv = pc.present && r - 1 >= pc.r0 && r - 1 <= pc.r1;
+                const int2 pr = *reinterpret_cast<const int2 *>(&cols[c - 1].r0);
+                po = r0 - pr.x;
+                prh = unsigned(pr.y - pr.x);
+                hc = ph[c - 1];
             }
-            const int hS = hv ? aS[k1 * cap + c - 1] : INF, hE = hv ? aE[k1 * cap + c - 1] : INF;
-            int kdS = INF, kvS = INF, kvF = INF;
-            if (cellk != CELL_FIRST) {
-                kvS = aS[k1 * cap + c];
-                kvF = aF[k1 * cap + c];
-                if (dv) kdS = aS[k2 * cap + c - 1];
-            } else if (cd.type != COL_INITIAL && (cd.loc == LOC_MIDDLE || cd.loc == LOC_BOTTOM) && r > 0 && dv) {
-                kdS = aS[k2 * cap + c - 1];
+            // (row 0 has no residue; its cells are given)
+            vc = r0 >= 1 ? vr[0] : 0;
+            vcNext = vr[1];
+            if (initial) {
+                given = vLeft[entry];
+                if (h > 0) givenNext = vLeft[entry + 1];
+            } else if (preset) {
+                given = vTop[entry];
             }
-            Cell cur{INF, INF, INF};
-            int tv = T_NONE;
-            const int cV = cd.vrow0 + dr, cH = cd.hcol;
-            if (cd.type == COL_INITIAL) {
-                const int idx = cV - (lp - 1);
-                if (idx < 0 || idx >= n4[1]) { fail(ST_UNDEFINED); continue; }
-                cur = w.v4[1][idx];
-            } else if (cellk == CELL_FIRST && (cd.loc == LOC_TOP || cd.loc == LOC_FULL)) {
-                if (cH >= n4[0]) { fail(ST_UNDEFINED); continue; }
-                cur = w.v4[0][cH];
-            } else {
-                const int dir = (cellk == CELL_INNER) ? DIR_ALL
-                              : (cellk == CELL_FIRST) ? DIR_UPPER
-                              : (cd.loc == LOC_TOP || cd.loc == LOC_MIDDLE) ? DIR_LOWER : DIR_ALL;
-                tv = compute(dir, c, r, hS, hE, cur, kdS, kvS, kvF);
+        };
+        if (c <= cend) enter();
+        int outS = INF, outE = INF;     // this lane's last cell, for the lane to its right
+        int upF = INF;                  // and for its own next cell (with outS)
+        int diagS = INF;                // what the left lane handed over one step ago
+        const int never = INT_MIN / 2;  // a lane without a column
+        int dr = c <= cend ? dlo - c - r0 : never;
+        for (int d = dlo; d <= dhi; ++d, ++dr) {
+            int leftS = __shfl_sync(0xffffffffu, outS, left);
+            int leftE = AFFINE ? __shfl_sync(0xffffffffu, outE, left) : INF;
+            const unsigned pr = unsigned(dr + po);                 // the row's place in the previous column
+            const bool act = unsigned(dr) <= unsigned(h);
+            const bool hv = pr <= prh && po != INT_MIN, dv = pr - 1u <= prh && po != INT_MIN;
+            if (carryIn && hv) {
+                leftS = cS[dr + r0];
+                leftE = cE[dr + r0];
             }
-            aS[k3 * cap + c] = cur.s;
-            aE[k3 * cap + c] = cur.e;
-            aF[k3 * cap + c] = cur.f;
-            w.T[p] = uint8_t(tv);
-            if (cH < hN) continue;
-            // the chain's tracking options
-            bool storeRow, lastCol = false, lastRow = false;
-            if (cd.loc == LOC_BOTTOM) storeRow = cV + lp == vN;
-            else storeRow = cV == vN;
-            const bool storeCol = cH == hN && cV >= vN;
-            if (cellk == CELL_LAST && (!finalM || freeB)) lastRow = true;
-            if (cd.type == COL_FINAL) {
-                if (cellk == CELL_LAST) { lastCol = true; lastRow = true; }
-                else if ((cd.loc != LOC_FULL || cV >= vN) && (!finalM || freeR)) lastCol = true;
+            // All directions, without the vertical one in a first cell (Upper) and without the
+            // horizontal one in the last cell of a top or middle column (Lower); the cells of the
+            // first column and the first cells of top and full columns are given.  No branches: a lane
+            // outside its column computes what nothing reads.
+            const bool vert = dr > 0, isLast = vert && dr == h, hori = !(isLast && lower);
+            const bool isGiven = initial || (!vert && preset);
+            const int hS = hv ? leftS : INF, hE = hv ? leftE : INF;
+            const int inter = (dv ? diagS : INF) + (hc == vc ? match : mismatch);
+            const int e1 = AFFINE ? hE + ext : hS + ext, e2 = AFFINE ? hS + open : e1;
+            const int f1 = AFFINE ? upF + ext : outS + ext, f2 = AFFINE ? outS + open : f1;
+            const int e = cmax(e1, e2), f = cmax(f1, f2);
+            const int eb = AFFINE ? (e1 >= e2 ? T_H : 0) | (e2 >= e1 ? T_HO : 0) : T_H;
+            const int fb = AFFINE ? (f1 >= f2 ? T_V : 0) | (f2 >= f1 ? T_VO : 0) : T_V;
+            const bool useF = vert && (!hori || f >= e), useE = hori && (!vert || e >= f);
+            const int g = useF ? f : e;
+            const int src = (useF ? T_MFV : 0) | (useE ? T_MFH : 0);
+            // affine cells keep both gaps' bits whichever direction wins, linear ones the winners' only
+            const int gaps = AFFINE ? (hori ? eb : 0) | (vert ? fb : 0) : (useE ? eb : 0) | (useF ? fb : 0);
+            int t_ = (inter >= g ? int(T_DIAG) : 0) | (g >= inter ? src : 0);
+            t_ |= AFFINE ? gaps : (g >= inter ? gaps : 0);
+            const int s_ = isGiven ? given.s : cmax(inter, g);
+            const int e_ = isGiven ? given.e : (AFFINE && hori ? e : INF);
+            const int f_ = isGiven ? given.f : (AFFINE && vert ? f : INF);
+            if (act) {
+                Tc[dr] = uint8_t(isGiven ? 0 : t_);
+                vc = vcNext;
+                vcNext = vr[dr + 2];   // loaded two rows ahead (the sequence buffers are padded)
             }
-            if (storeCol) {
-                const int q = cV - vN;
-                if (q >= n4[3]) { fail(ST_UNDEFINED); continue; }
-                w.v4[3][q] = cur;
+            outS = act ? s_ : outS;
+            outE = act ? e_ : outE;
+            upF = act ? f_ : upF;
+            if (initial && act) {
+                given = givenNext;
+                if (dr + 1 < h) givenNext = vLeft[entry + dr + 2];
             }
-            if (storeRow) {
-                const int q = cH - hN;
-                if (q >= n4[2]) { fail(ST_UNDEFINED); continue; }
-                w.v4[2][q] = cur;
+            if (carryOut && act) {
+                cS[dr + r0] = s_;
+                cE[dr + r0] = e_;
             }
-            if (lastCol || lastRow) {
-                if (cd.type == COL_FINAL) {
-                    w.fcS[r] = cur.s;
-                    w.fcP[r] = p;
-                    w.fcF[r] = 1;
-                } else {
-                    w.ccS[c] = cur.s;
-                    w.ccP[c] = p;
-                    w.ccF[c] = 1;
+            if (act && dr + r0 >= rowAny) {
+                const int r = dr + r0;
+                if (r >= rowCol) outCol[r - rowCol] = Cell{s_, e_, f_};
+                if (r == rowStore) outRow[initial ? 0 : entry - stored] = Cell{s_, e_, f_};
+                if (r >= rowTrack) {
+                    if (kind_ & CD_FINAL) {
+                        fcS[r] = s_;
+                        fcP[r] = int(Tc - T) + dr;
+                    } else {
+                        cols[c].candS = s_;
+                        cols[c].candP = int(Tc - T) + dr;
+                    }
                 }
             }
+            diagS = leftS;
+            if (wrap && dr == h && c + 32 <= cend) {
+                c += 32;
+                enter();
+                dr = d - c - r0;
+            }
         }
     }
 
-    __host__ __device__ void offer_chain(int s_, int p_)
+    // Appends the candidates of value maxS that the lanes hold (position < 0: none), in lane order.
+    GBA_CHAIN_STEP __device__ void collect(int s_, int p_)
     {
-        if (s_ >= maxS) {
-            if (s_ != maxS) { nmp = 0; maxS = s_; }
-            if (nmp >= pl->mp_cap) { fail(ST_CAPACITY); return; }
-            w.mp[nmp++] = p_;
-        }
+        const int lane = lane_id();
+        const bool mine = p_ >= 0 && s_ == maxS;
+        const unsigned who = __ballot_sync(0xffffffffu, mine);
+        if (nmp + __popc(who) > pl->mp_cap) { fail(ST_CAPACITY); return; }
+        if (mine) w.mp[nmp + __popc(who & ((1u << lane) - 1u))] = p_;
+        const int n = nmp + __popc(who);
+        __syncwarp();
+        nmp = n;
+        __syncwarp();
     }
 
-    __host__ __device__ void fill_warp()
+    __device__ void fill_warp()
     {
         if (gm + 1 > pl->col_cap || gn + 1 > pl->col_rows) { fail(ST_CAPACITY); return; }
-        const int64_t cells = L * Hlen;
-#ifdef __CUDA_ARCH__
-        for (int64_t q = lane; q < cells; q += 32) w.T[q] = 0;
-        for (int c = lane; c <= gm; c += 32) { w.cols[c].present = 0; w.ccF[c] = 0; }
-        for (int r = lane; r <= gn; r += 32) w.fcF[r] = 0;
-        __syncwarp();
-#else
-        for (int64_t q = 0; q < cells; ++q) w.T[q] = 0;
-        for (int c = 0; c <= gm; ++c) { w.cols[c].present = 0; w.ccF[c] = 0; }
-        for (int r = 0; r <= gn; ++r) w.fcF[r] = 0;
-#endif
+        const int lane = lane_id();
+        for (int r = lane; r <= gn; r += 32) w.fcP[r] = -1;
         int cfirst = 0, clast = 0;
-        describe(cfirst, clast);   // every lane writes the same descriptors
-#ifdef __CUDA_ARCH__
+        describe(cfirst, clast);
         __syncwarp();
-#endif
         if (err) return;
-        int64_t dmin = INT64_MAX, dmax = -1;
-        for (int c = cfirst; c <= clast; ++c) {
-            const ColDesc &cd = w.cols[c];
-            if (!cd.present) continue;
-            dmin = cmin<int64_t>(dmin, int64_t(c) + cd.r0);
-            dmax = cmax<int64_t>(dmax, int64_t(c) + cd.r1);
+        int dlo = INT_MAX, dhi = -1;
+        bool wrap = true;
+        for (int c = cfirst + lane; c <= clast; c += 32) {
+            dlo = cmin(dlo, c + w.cols[c].r0);
+            dhi = cmax(dhi, c + w.cols[c].r1);
+            wrap = wrap && (c + 32 > clast || w.cols[c].r1 < 32 + w.cols[c + 32].r0);
         }
-        int k3 = int(dmin % 3), k1 = (k3 + 2) % 3, k2 = (k3 + 1) % 3;
-        for (int d = int(dmin); d <= int(dmax); ++d) {
-#ifdef __CUDA_ARCH__
-            fill_diag(d, lane, cfirst, clast, k3, k1, k2);
-            __syncwarp();
-#else
-            for (int l = 0; l < 32; ++l) fill_diag(d, l, cfirst, clast, k3, k1, k2);
-#endif
-            const int t = k2;   // d + 1: its d - 1 is this d, its d - 2 this d - 1
-            k2 = k1;
-            k1 = k3;
-            k3 = t;
-        }
-#ifdef __CUDA_ARCH__
-        err = __reduce_max_sync(0xffffffffu, err);
-#endif
-        if (err) return;
-        // the scout's positions of the maximum, in the loop's order
-        for (int c = cfirst; c <= clast && !err; ++c) {
-            const ColDesc &cd = w.cols[c];
-            if (!cd.present) continue;
-            if (cd.type == COL_FINAL) {
-                for (int r = cd.r0; r <= cd.r1; ++r)
-                    if (w.fcF[r]) offer_chain(w.fcS[r], w.fcP[r]);
-            } else if (w.ccF[c]) {
-                offer_chain(w.ccS[c], w.ccP[c]);
+        wrap = __all_sync(0xffffffffu, wrap);
+        if (wrap) {
+            const int lo = __reduce_min_sync(0xffffffffu, dlo), hi = __reduce_max_sync(0xffffffffu, dhi);
+            if (affine) sweep<true>(cfirst, cfirst, clast, true, lo, hi);
+            else sweep<false>(cfirst, cfirst, clast, true, lo, hi);
+        } else {
+            for (int c0 = cfirst; c0 <= clast; c0 += 32) {
+                const int c = c0 + lane, ce = cmin(clast, c0 + 31);
+                const int lo = __reduce_min_sync(0xffffffffu, c <= ce ? c + w.cols[c].r0 : INT_MAX);
+                const int hi = __reduce_max_sync(0xffffffffu, c <= ce ? c + w.cols[c].r1 : -1);
+                if (affine) sweep<true>(cfirst, c0, ce, false, lo, hi);
+                else sweep<false>(cfirst, c0, ce, false, lo, hi);
+                __syncwarp();
             }
         }
+        __syncwarp();
+        if (err) return;
+        // the scout's positions of the maximum, in the loop's order
+        const bool tail = (w.cols[clast].kind & CD_FINAL) != 0;   // the final column's candidates are per row
+        const int t0 = tail ? w.cols[clast].r0 : 0, t1 = tail ? w.cols[clast].r1 : -1;
+        int best = INT_MIN;
+        for (int c = cfirst + lane; c <= clast; c += 32)
+            if (w.cols[c].candP >= 0) best = cmax(best, w.cols[c].candS);
+        for (int r = t0 + lane; r <= t1; r += 32)
+            if (w.fcP[r] >= 0) best = cmax(best, w.fcS[r]);
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (best < maxS) return;
+        __syncwarp();
+        maxS = best;
+        __syncwarp();
+        for (int c0 = cfirst; c0 <= clast && !err; c0 += 32) {
+            const int c = c0 + lane;
+            collect(c <= clast ? w.cols[c].candS : 0, c <= clast ? w.cols[c].candP : -1);
+        }
+        for (int r0 = t0; r0 <= t1 && !err; r0 += 32) {
+            const int r = r0 + lane;
+            collect(r <= t1 ? w.fcS[r] : 0, r <= t1 ? w.fcP[r] : -1);
+        }
+        __syncwarp();
     }
+#else
+    __host__ void fill_warp() { fail(ST_UNDEFINED); }   // the host runs the geometry only
+#endif
 
     // ---------------- the chain driver ----------------
     struct Seed { int64_t bh, bv, eh, ev, lo, up; };
@@ -1484,6 +1614,17 @@ struct Engine {
     }
 };
 
+// A warp's part of the block's shared memory.  The engine is one per warp: its lanes run the driver,
+// the tracebacks and the glue in lockstep on the same values (every lane writes what the others
+// write), and 32 private copies of its state overflowed L1.
+struct WarpShared {
+    uint8_t T[kSharedTrace];
+    ColDesc cols[kSharedCols];
+    Engine engine;
+    Plan plan;
+};
+constexpr size_t kSharedPerWarp = (sizeof(WarpShared) + 15) & ~size_t(15);
+
 }  // namespace chain
 
 struct ChainArgs {
@@ -1495,6 +1636,7 @@ struct ChainArgs {
     chain::Scheme anchor, gap;
     int32_t free_ends, band_ext, affine, max_traces;
     int32_t *score, *status, *n_traces, *seg_count;
+    int32_t *next;                    // work counter, zeroed before the launch
 };
 
 namespace chain {
@@ -1522,18 +1664,11 @@ __host__ __device__ inline int64_t layout(const Plan &p, int max_traces, uint8_t
     int *llen = reinterpret_cast<int *>(take(int64_t(max_traces) * 4));
     int *erase = reinterpret_cast<int *>(take(int64_t(max_traces) * 4));
     ColDesc *cols = reinterpret_cast<ColDesc *>(take(int64_t(p.col_cap) * int64_t(sizeof(ColDesc))));
-    int *aS = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 12));
-    int *aE = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 12));
-    int *aF = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 12));
-    int *ccS = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 4));
-    int *ccP = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 4));
-    int *ccF = reinterpret_cast<int *>(take(int64_t(p.col_cap) * 4));
     int *fcS = reinterpret_cast<int *>(take(int64_t(p.col_rows) * 4));
     int *fcP = reinterpret_cast<int *>(take(int64_t(p.col_rows) * 4));
-    int *fcF = reinterpret_cast<int *>(take(int64_t(p.col_rows) * 4));
     if (w) {
-        w->cols = cols; w->aS = aS; w->aE = aE; w->aF = aF;
-        w->ccS = ccS; w->ccP = ccP; w->ccF = ccF; w->fcS = fcS; w->fcP = fcP; w->fcF = fcF;
+        w->cols = w->arenaCols = cols; w->fcS = fcS; w->fcP = fcP;
+        w->arenaT = T;
         w->T = T; w->cS0 = c0; w->cS1 = c1; w->cE0 = e0; w->cE1 = e1;
         for (int q = 0; q < 4; ++q) w->v4[q] = v4[q];
         w->set = set; w->mp = mp; w->gseg = gseg; w->glen = glen; w->gorder = gorder;
@@ -1550,38 +1685,51 @@ void launch_chain_pack(const chain::ChainDesc *chains, int64_t num_chains, const
                        const int32_t *seg_count, const int64_t *dense_off, chain::Seg *dense, cudaStream_t st);
 
 #ifdef SEQAN_GB300_CHAIN_KERNELS
-__global__ void __launch_bounds__(128) k_banded_chain(ChainArgs a)
+// Persistent: a warp takes the next chain (longest first) when it is done with one.
+__global__ void __launch_bounds__(128, 4) k_banded_chain(ChainArgs a)
 {
-    const int64_t c = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = int(threadIdx.x & 31);
-    if (c >= a.num_chains) return;   // whole warps leave together
-    const chain::ChainDesc &d = a.chains[c];
-    chain::Plan pl = d.plan;
-    chain::Engine e;
-    e.plan = false;
-    e.warp = true;
-    e.lane = lane;
-    e.anchor = a.anchor;
-    e.gap = a.gap;
-    e.fe = a.free_ends;
-    e.affine = a.affine;
-    e.k = a.band_ext;
-    e.max_traces = a.max_traces;
-    e.h = a.seq_h + d.h_off;
-    e.v = a.seq_v + d.v_off;
-    e.m = d.m;
-    e.n = d.n;
-    e.pl = &pl;
-    chain::layout(pl, a.max_traces, a.arena + d.arena_off, &e.w);
-    int score = INT_MIN;
-    if (pl.status == chain::ST_OK) score = e.run(a.seeds + 4 * d.seed_off, d.n_seeds);
-    else e.err = pl.status;
-    __syncwarp();
-    if (lane == 0) {
-        a.score[c] = score;
-        a.status[c] = e.err;
-        a.n_traces[c] = e.ng;
-        a.seg_count[c] = (!e.err && e.ng > 0) ? e.w.glen[e.w.gorder[0]] : 0;
+    extern __shared__ uint4 chain_shared[];
+    chain::WarpShared &ws = *reinterpret_cast<chain::WarpShared *>(
+        reinterpret_cast<uint8_t *>(chain_shared) + (threadIdx.x >> 5) * chain::kSharedPerWarp);
+    chain::Engine &e = ws.engine;
+    for (;;) {
+        int c = 0;
+        if (lane == 0) c = atomicAdd(a.next, 1);
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= a.num_chains) return;
+        const chain::ChainDesc &d = a.chains[c];
+        ws.plan = d.plan;
+        e.plan = false;
+        e.warp = true;
+        e.anchor = a.anchor;
+        e.gap = a.gap;
+        e.fe = a.free_ends;
+        e.affine = a.affine;
+        e.k = a.band_ext;
+        e.max_traces = a.max_traces;
+        e.h = a.seq_h + d.h_off;
+        e.v = a.seq_v + d.v_off;
+        e.m = d.m;
+        e.n = d.n;
+        e.pl = &ws.plan;
+        e.ng = 0;
+        chain::layout(ws.plan, a.max_traces, a.arena + d.arena_off, &e.w);
+        e.w.sharedT = ws.T;
+        e.w.sharedCols = ws.cols;
+        const int status = ws.plan.status;
+        __syncwarp();
+        int score = INT_MIN;
+        if (status == chain::ST_OK) score = e.run(a.seeds + 4 * d.seed_off, d.n_seeds);
+        else e.err = status;
+        __syncwarp();
+        if (lane == 0) {
+            a.score[d.id] = score;
+            a.status[d.id] = e.err;
+            a.n_traces[d.id] = e.ng;
+            a.seg_count[d.id] = (!e.err && e.ng > 0) ? e.w.glen[e.w.gorder[0]] : 0;
+        }
+        __syncwarp();
     }
 }
 
@@ -1594,13 +1742,13 @@ __global__ void __launch_bounds__(128) k_chain_pack(const chain::ChainDesc *chai
 {
     const int64_t c = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (c >= num_chains) return;
-    const int32_t cnt = seg_count[c];
-    if (cnt <= 0) return;
     const chain::ChainDesc &d = chains[c];
+    const int32_t cnt = seg_count[d.id];
+    if (cnt <= 0) return;
     chain::Work w;
     chain::layout(d.plan, max_traces, const_cast<uint8_t *>(arena) + d.arena_off, &w);
     const chain::Seg *src = w.gseg + int64_t(w.gorder[0]) * d.plan.gseg_cap;
-    chain::Seg *dst = dense + dense_off[c];
+    chain::Seg *dst = dense + dense_off[d.id];
     for (int32_t q = 0; q < cnt; ++q) dst[q] = src[cnt - 1 - q];
 }
 #endif
