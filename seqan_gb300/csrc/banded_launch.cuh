@@ -3,6 +3,7 @@
 // parallel: the register form of the kernel is the largest code in the engine.
 #pragma once
 
+#include "dp_banded2_kernels.cuh"
 #include "dp_banded_kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -17,6 +18,9 @@ BandLauncher pick_banded_affine_global(bool matrix, bool trace);
 BandLauncher pick_banded_affine_local(bool matrix, bool trace);
 BandLauncher pick_banded_linear_global(bool matrix, bool trace);
 BandLauncher pick_banded_linear_local(bool matrix, bool trace);
+// The two-pairs-per-thread instances (global units): grid in blocks of kLaunchBlock threads.
+BandLauncher pick_banded2_affine(bool matrix, bool trace);
+BandLauncher pick_banded2_linear(bool matrix, bool trace);
 BandLauncher pick_banded_ext_affine(bool matrix, bool trace);
 BandLauncher pick_banded_ext_linear(bool matrix, bool trace);
 
@@ -36,6 +40,20 @@ void launch(const BandArgs &args, int grid, size_t smem, cudaStream_t s)
         k_dp_banded<A, L, M, T, kSmallBandWidth, XT><<<grid, kLaunchBlock, smem, s>>>(args);
     else
         k_dp_banded<A, L, M, T, kMaxBandSlots, XT><<<grid, kLaunchBlock, smem, s>>>(args);
+}
+
+template <bool A, bool M, bool T>
+void launch2(const BandArgs &args, int grid, size_t smem, cudaStream_t s)
+{
+    k_dp_banded2<A, M, T><<<grid, kLaunchBlock, smem, s>>>(args);
+}
+
+template <bool A>
+BandLauncher pick2(bool m, bool t)
+{
+    static const BandLauncher table[4] = {launch2<A, false, false>, launch2<A, false, true>, launch2<A, true, false>,
+                                          launch2<A, true, true>};
+    return table[(m ? 2 : 0) | (t ? 1 : 0)];
 }
 
 template <bool A, bool L, bool XT>

@@ -7,4 +7,6 @@ BandLauncher pick_banded_affine_global(bool m, bool t) { return banded_launch::p
 
 BandLauncher pick_banded_ext_affine(bool m, bool t) { return banded_launch::pick<true, false, true>(m, t); }
 
+BandLauncher pick_banded2_affine(bool m, bool t) { return banded_launch::pick2<true>(m, t); }
+
 }  // namespace gba

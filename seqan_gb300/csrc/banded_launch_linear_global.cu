@@ -7,4 +7,6 @@ BandLauncher pick_banded_linear_global(bool m, bool t) { return banded_launch::p
 
 BandLauncher pick_banded_ext_linear(bool m, bool t) { return banded_launch::pick<false, false, true>(m, t); }
 
+BandLauncher pick_banded2_linear(bool m, bool t) { return banded_launch::pick2<false>(m, t); }
+
 }  // namespace gba

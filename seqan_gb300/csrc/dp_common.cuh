@@ -56,7 +56,8 @@ struct PairDesc {
     int32_t n;           // |V| (rows)
     int32_t inf;         // DPCellDefaultInfinity of the cell width the pair runs with
     int16_t invalid;     // 1: empty sequence or band outside the matrix (score = numeric min)
-    int16_t rows;        // packed 16-bit warp kernel: rows per strip
+    int16_t rows;        // packed 16-bit warp kernel: rows per strip; banded: 1 / 2 the low / high pair
+                         // of a thread that runs two, 0 alone
 };
 
 // Arguments of the DP kernels, passed by value.

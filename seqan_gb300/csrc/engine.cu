@@ -83,6 +83,7 @@ struct gba_plan {
     // host side
     int64_t num_pairs = 0;
     int64_t num_slots = 0;          // valid pairs
+    int64_t duo_slots = 0;          // slots of banded pairs two to a thread (groups of 64, ahead of the others)
     bool traceback = false;
     bool cigar = false;
     bool affine = false;
@@ -241,6 +242,7 @@ BandLauncher pick_banded(bool a, bool l, bool m, bool t)
     return a ? (l ? pick_banded_affine_local(m, t) : pick_banded_affine_global(m, t))
              : (l ? pick_banded_linear_local(m, t) : pick_banded_linear_global(m, t));
 }
+BandLauncher pick_banded2(bool a, bool m, bool t) { return a ? pick_banded2_affine(m, t) : pick_banded2_linear(m, t); }
 BandLauncher pick_banded_ext(bool a, bool m, bool t)
 {
     return a ? pick_banded_ext_affine(m, t) : pick_banded_ext_linear(m, t);
@@ -359,6 +361,16 @@ bool w2_fits(const gba_params &p, int max_pos, int64_t m, int64_t n, bool local)
     const int64_t open = -int64_t(p.gap_open), ext = -int64_t(p.gap_extend);
     if (int64_t(max_pos) * (std::min(m, n) + 64) > 32767 - 64) return false;
     return local || -(3 * open + ext * (m + n + 66)) > kW2Inf + 2 * (open + ext) + 64;
+}
+
+// True when an m x n banded pair's values stay in the range of the two-pairs-per-thread banded kernel:
+// a cell's score is at least its diagonal's from the border (substitutions of at least -neg), and at
+// most max_pos per residue.
+bool band2_fits(const gba_params &p, int max_pos, int neg, int64_t m, int64_t n)
+{
+    const int64_t open = -int64_t(p.gap_open), ext = -int64_t(p.gap_extend), k = std::min(m, n);
+    return m < 65536 && n < 65536 && max_pos * k <= kBand2Max &&
+           -(3 * open + ext * (m + n + 2) + neg * k) >= kBand2Min;
 }
 
 // Rows per strip (2, 3, 4, 5, 6 or 8) that cover n rows in `bands` bands.
@@ -627,7 +639,7 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     plan->matrix_host.clear();
     if (p->matrix) plan->matrix_host.assign(p->matrix, p->matrix + p->alphabet_size * p->alphabet_size);
     int max_pos = 0;
-    max_sub_abs(*p, plan->matrix_host, &max_pos);
+    const int max_abs = max_sub_abs(*p, plan->matrix_host, &max_pos);
 
     plan->status.assign(N, GBA_PAIR_OK);
     // The packed 16-bit path: global score-only runs with equality scoring over an alphabet of
@@ -663,6 +675,13 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
                 p->mismatch >= -128 && p->mismatch <= 127;
     }
     const bool w2_narrow = (p->flags & GBA_FLAG_WARP16) != 0;
+    // The two-pairs-per-thread banded kernel: global alignments in bands of 2 to kBandFastW diagonals.
+    const int band_w = p->band_on ? p->band_upper - p->band_lower + 1 : 0;
+    const bool band2_ok = band_w >= 2 && band_w <= kBandFastW && !plain && !plan->local && !plan->extend &&
+                          !(p->flags & GBA_FLAG_GENERAL_KERNEL) && p->gap_open <= 0 && p->gap_extend <= 0 &&
+                          p->gap_open >= -1024 && p->gap_extend >= -1024 && max_abs <= 1024 &&
+                          (plan->matrix || (p->alphabet_size >= 1 && p->alphabet_size <= 8 && p->match >= -128 &&
+                                            p->match <= 127 && p->mismatch >= -128 && p->mismatch <= 127));
     const int w2_most = w2_max_rows(plan->w2_mat, plan->local, plan->traceback);
     // Host arrays live in the plan and keep their capacity between builds (no zero fill).
     auto &keys16 = plan->h_keys16;
@@ -756,6 +775,8 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
                 key[k] = uint32_t(std::min<int64_t>(strips * (d.m + 1), 0xffffffffLL));
                 cls[k] = 2;
                 ++not16;
+                // (rows: 1 marks a pair that may share a thread until the pairing below)
+                if (band2_ok && band2_fits(*p, max_pos, max_abs, d.m, d.n)) d.rows = 1;
             }
             if (plan->traceback) {
                 tbytes[k] = p->band_on ? int64_t(d.m + 1) * band_col_bytes(p->band_upper - p->band_lower + 1) / 32
@@ -834,27 +855,96 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
         sort_desc(keys, idx);
     }
     plan->num_slots = int64_t(idx.size());
-    // Banded traces are interleaved by lane within each warp of 32 slots (see band_trace_pos and
-    // band4_pos): a warp's region holds (its largest m + 1) columns of band_col_bytes(W) bytes
-    // for the 32 lanes, rounded up to 512 bytes so that a pair's lane is (trace_off >> 4) & 31.
+    // Banded pairs of equal |H| and |V| share a thread two by two (dp_banded2_kernels.cuh): slots in
+    // groups of 64, thread l of a warp holding slots l and 32 + l.  The other pairs follow, one a thread.
+    plan->duo_slots = 0;
+    if (band2_ok && !idx.empty()) {
+        int64_t fit = 0;
+        int32_t m0 = INT32_MAX, m1 = 0, n0 = INT32_MAX, n1 = 0;
+        for (int32_t k : idx)
+            if (desc[k].rows) {
+                ++fit;
+                m0 = std::min(m0, desc[k].m);
+                m1 = std::max(m1, desc[k].m);
+                n0 = std::min(n0, desc[k].n);
+                n1 = std::max(n1, desc[k].n);
+            }
+        std::vector<int32_t> duo, rest;
+        duo.reserve(size_t(fit));
+        rest.reserve(idx.size() - size_t(fit) + 64);
+        for (int32_t k : idx) (desc[k].rows ? duo : rest).push_back(k);
+        if (m0 < m1 || n0 < n1) {
+            const uint32_t span = uint32_t(n1 - n0 + 1);
+            std::vector<uint32_t> dk(duo.size());
+            for (size_t i = 0; i < duo.size(); ++i) dk[i] = uint32_t(desc[duo[i]].m - m0) * span + uint32_t(desc[duo[i]].n - n0);
+            sort_desc(dk, duo);
+        }
+        auto same = [&](int32_t x, int32_t y) { return desc[x].m == desc[y].m && desc[x].n == desc[y].n; };
+        // neighbours of one size make a duo; an odd one out goes with the rest
+        std::vector<int32_t> lo, hi;
+        lo.reserve(duo.size() / 2 + 32);
+        hi.reserve(duo.size() / 2 + 32);
+        for (size_t i = 0; i < duo.size();) {
+            if (i + 1 < duo.size() && same(duo[i], duo[i + 1])) {
+                lo.push_back(duo[i]);
+                hi.push_back(duo[i + 1]);
+                i += 2;
+            } else {
+                desc[duo[i]].rows = 0;
+                rest.push_back(duo[i++]);
+            }
+        }
+        lo.resize((lo.size() + 31) / 32 * 32, -1);
+        hi.resize(lo.size(), -1);
+        plan->duo_slots = int64_t(lo.size()) * 2;
+        idx.resize(size_t(plan->duo_slots) + rest.size());
+#pragma omp parallel for num_threads(plan_threads(plan->duo_slots)) schedule(static)
+        for (int64_t q = 0; q < int64_t(lo.size()); ++q) {
+            const int64_t at = q / 32 * 64 + q % 32;
+            idx[at] = lo[q];
+            idx[at + 32] = hi[q];
+            if (lo[q] >= 0) {
+                desc[lo[q]].rows = 1;      // low half
+                desc[hi[q]].rows = 2;      // high half
+            }
+        }
+        std::copy(rest.begin(), rest.end(), idx.begin() + plan->duo_slots);
+        plan->num_slots = int64_t(idx.size());
+    }
+    // Banded traces are interleaved by lane within each warp: a warp's region holds (its largest
+    // m + 1) columns of band2_col_bytes(W) bytes for its 64 pairs, or of band_col_bytes(W) for its 32
+    // (band_trace_pos, band4_pos), rounded up to 512 bytes so that a pair's lane is
+    // (trace_off >> 4) & 31.
     if (p->band_on && plan->traceback && plan->num_slots > 0) {
-        const int CB = band_col_bytes(p->band_upper - p->band_lower + 1);
-        const int64_t nw = (plan->num_slots + 31) / 32;
+        const int64_t nd = plan->duo_slots / 64, nw = nd + (plan->num_slots - plan->duo_slots + 31) / 32;
         std::vector<int64_t> wsize(nw + 1, 0);
+        auto range = [&](int64_t w, int64_t &s0, int64_t &s1, int &CB) {
+            CB = w < nd ? band2_col_bytes(band_w) : band_col_bytes(band_w);
+            s0 = w < nd ? 64 * w : plan->duo_slots + 32 * (w - nd);
+            s1 = std::min(plan->num_slots, s0 + (w < nd ? 64 : 32));
+        };
 #pragma omp parallel for num_threads(plan_threads(plan->num_slots)) schedule(static)
         for (int64_t w = 0; w < nw; ++w) {
-            int maxm = -1;
-            for (int64_t s = 32 * w; s < std::min(plan->num_slots, 32 * w + 32); ++s)
+            int maxm = -1, CB = 0;
+            int64_t s0, s1;
+            range(w, s0, s1, CB);
+            for (int64_t s = s0; s < s1; ++s)
                 if (idx[s] >= 0) maxm = std::max(maxm, desc[idx[s]].m);
             wsize[w + 1] = maxm < 0 ? 0 : (int64_t(maxm + 1) * CB + 511) / 512 * 512;
         }
         for (int64_t w = 0; w < nw; ++w) wsize[w + 1] += wsize[w];
 #pragma omp parallel for num_threads(plan_threads(plan->num_slots)) schedule(static)
-        for (int64_t s = 0; s < plan->num_slots; ++s)
-            if (idx[s] >= 0) desc[idx[s]].trace_off = wsize[s / 32] + (s % 32) * 16;
+        for (int64_t w = 0; w < nw; ++w) {
+            int CB = 0;
+            int64_t s0, s1;
+            range(w, s0, s1, CB);
+            for (int64_t s = s0; s < s1; ++s)
+                if (idx[s] >= 0) desc[idx[s]].trace_off = wsize[w] + ((s - s0) % 32) * 16;
+        }
         trace_off = wsize[nw];
         plan->trace_total = trace_off;
     }
+
     // Packed path: neighbours in the length-sorted order share a thread; per warp, the code
     // words (4 residues per word, both pairs' codes per byte) and the boundary row are
     // interleaved by lane.
@@ -1513,14 +1603,24 @@ int enqueue_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const 
         b.upper = plan->params.band_upper;
         b.xdrop_on = plan->extend && (plan->params.flags & GBA_FLAG_XDROP) ? 1 : 0;
         b.xdrop = plan->params.xdrop;
-        const int grid = int((plan->num_slots + kBlock - 1) / kBlock);
         const size_t smem = plan->matrix ? size_t(32 * 32) * sizeof(int) : 0;
-        if (plan->extend)
-            pick_banded_ext(plan->affine, plan->matrix, plan->traceback)(b, grid, smem, ctx->stream);
-        else
-            pick_banded(plan->affine, plan->local, plan->matrix, plan->traceback)(b, grid, smem, ctx->stream);
+        if (plan->duo_slots > 0) {
+            BandArgs b2 = b;
+            b2.num_slots = plan->duo_slots;
+            pick_banded2(plan->affine, plan->matrix, plan->traceback)(b2, warp_blocks(plan->duo_slots / 64), smem, ctx->stream);
+            ++launches;
+        }
+        if (plan->num_slots > plan->duo_slots) {
+            b.order += plan->duo_slots;
+            b.num_slots -= plan->duo_slots;
+            const int grid = int((b.num_slots + kBlock - 1) / kBlock);
+            if (plan->extend)
+                pick_banded_ext(plan->affine, plan->matrix, plan->traceback)(b, grid, smem, ctx->stream);
+            else
+                pick_banded(plan->affine, plan->local, plan->matrix, plan->traceback)(b, grid, smem, ctx->stream);
+            ++launches;
+        }
         GBA_CUDA(ctx, cudaGetLastError());
-        ++launches;
     } else if (plan->num_slots > 0 && plan->use_warp) {
         WarpArgs w{};
         w.seq_h = dseq_h;

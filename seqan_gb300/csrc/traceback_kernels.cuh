@@ -16,6 +16,7 @@
 #pragma once
 
 #include "dp_common.cuh"
+#include "dp_banded2_kernels.cuh"
 #include "dp_banded_kernels.cuh"
 #include "dp_warp_kernels.cuh"
 #include "dp_warp2_kernels.cuh"
@@ -241,6 +242,8 @@ __global__ void __launch_bounds__(128) k_traceback(TraceArgs a)
     const int bw = a.band_w, bu = a.band_upper;
     const bool affine = a.affine != 0;
     auto TAT = [&](int c, int r) -> int {
+        if (bw && d.rows)   // two pairs a thread
+            return int(trace_at_band2(T, int((d.trace_off >> 4) & 31), d.rows - 1, bw, bu, affine, c, r));
         return bw ? int(trace_at_band(T, d.trace_off, bw, bu, affine, c, r)) : int(trace_at(T, m, c, r));
     };
     LaneSteps<decltype(TAT)> steps{TAT};
