@@ -17,6 +17,7 @@
 #include "dp_dynamic_kernels.cuh"
 #include "seed_kernels.cuh"
 #include "extend_kernels.cuh"
+#include "extend2_kernels.cuh"
 #include "int_peak.cuh"
 
 #include <cub/device/device_scan.cuh>
@@ -225,7 +226,8 @@ struct gba_context {
     bool xs_check = false;          // a device seed-extension run whose error word is unread
     std::map<std::pair<const void *, size_t>, int64_t> xs_grid;   // (kernel, smem) -> resident blocks
     // alignment extension: tasks, per-task results, trace, segments, scratch
-    DevBuf xa_tasks, xa_out, xa_trace, xa_segs, xa_segoff, xa_segcnt, xa_scratch, xa_next, xa_packoff, xa_packed;
+    DevBuf xa_tasks, xa_out, xa_trace, xa_segs, xa_segoff, xa_segcnt, xa_scratch, xa_next, xa_packoff, xa_packed,
+        xa_seeds, xa_off_h, xa_off_v, xa_ids, xa_tmp, xa_scores;
     DevBuf en_pairs, en_mat, en_forb, en_heap, en_steps, en_slots, en_out, en_dense, en_offs, en_cnt;   // gba_local_enumerate
     DevBuf bc_seeds, bc_desc, bc_arena, bc_out, bc_dense, bc_offs;   // gba_banded_chain
     DevBuf bz_in, bz_slots, bz_scratch, bz_meta, bz_out;             // gba_bgzf_compress

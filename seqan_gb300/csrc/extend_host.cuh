@@ -1,8 +1,9 @@
 // extend_host.cuh -- host side of gba_extend_alignments (included at the end of engine.cu).
 //
 // Each alignment contributes up to two tasks (its left side on the reversed prefixes, its right
-// side on the suffixes).  A score pass runs the AlignExtend DP with the X-drop terminator and
-// finds each task's best cell and last computed column; the host then sizes the trace
+// side on the suffixes).  Batches of many sides whose values fit 16 bits run two sides per thread in
+// one pass (ext_paired).  For the others a score pass runs the AlignExtend DP with the X-drop
+// terminator and finds each task's best cell and last computed column; the host then sizes the trace
 // (last column + 1 columns of round8(rows + 1) bytes per task) and the segment slots, and a trace
 // pass recomputes exactly those columns with trace, followed by the traceback.  Tasks are cut
 // into chunks whose trace fits kExtTraceBudget.  With a band, both sides run as one
@@ -206,6 +207,290 @@ int ext_banded(gba_context *ctx, const gba_extend_align_params *params, const st
     return GBA_OK;
 }
 
+constexpr int64_t kX2MinSides = 512;
+constexpr int kX2Most = 1024;                    // scores and gap costs, and rows of a side
+constexpr int kX2MostCols = 4096;
+
+// The sides of a batch: their number, sizes and cells.
+struct ExtSides {
+    int64_t count = 0, mmax = 0, nmax = 0, cells = 0;
+    bool valid = true;
+    std::vector<int32_t> m, n;       // by id = 2 * alignment + side; 0: no extension there
+};
+
+ExtSides ext_sides(const gba_extend_align_params *p, const gba_seed_batch *b, const gba_seed *seeds)
+{
+    ExtSides x;
+    const int64_t ns = b->num_seeds;
+    x.m.resize(size_t(ns) * 2);
+    x.n.resize(size_t(ns) * 2);
+    int64_t count = 0, mmax = 0, nmax = 0, bad = 0, cells = 0;
+#pragma omp parallel for num_threads(plan_threads(ns)) schedule(static) reduction(+ : count, bad, cells) reduction(max : mmax, nmax)
+    for (int64_t k = 0; k < ns; ++k) {
+        const int64_t hi = b->seed_h ? b->seed_h[k] : k, vi = b->seed_v ? b->seed_v[k] : k;
+        if (hi < 0 || hi >= b->num_h || vi < 0 || vi >= b->num_v) { ++bad; continue; }
+        const int64_t lh = b->off_h[hi + 1] - b->off_h[hi], lv = b->off_v[vi + 1] - b->off_v[vi];
+        const gba_seed &s = seeds[k];
+        if (lh > kExtMaxLen || lv > kExtMaxLen ||
+            !(0 <= s.begin_h && s.begin_h <= s.end_h && s.end_h <= lh && 0 <= s.begin_v && s.begin_v <= s.end_v &&
+              s.end_v <= lv)) { ++bad; continue; }
+        const bool on[2] = {(p->direction & GBA_EXTEND_LEFT) && s.begin_h > 0 && s.begin_v > 0,
+                            (p->direction & GBA_EXTEND_RIGHT) && s.end_h < lh && s.end_v < lv};
+        for (int side = 0; side < 2; ++side) {
+            const int64_t m = !on[side] ? 0 : side ? lh - s.end_h : s.begin_h;
+            const int64_t n = !on[side] ? 0 : side ? lv - s.end_v : s.begin_v;
+            x.m[2 * k + side] = int32_t(m);
+            x.n[2 * k + side] = int32_t(n);
+            count += on[side];
+            cells += m * n;
+            mmax = std::max(mmax, m);
+            nmax = std::max(nmax, n);
+        }
+    }
+    x.count = count;
+    x.mmax = mmax;
+    x.nmax = nmax;
+    x.cells = cells;
+    x.valid = bad == 0;
+    return x;
+}
+
+// True when two sides per thread is the form for a batch: gaps cost something (the best cell then
+// never ends in one), values fit 16 bits, and the time expected is the shorter.  A thread takes
+// 0.46 us per column of a strip and has the whole side to itself; trace chunks follow one another.
+// A group of lanes takes 4 us per column (both passes), so it is done first with a few sides, but
+// costs 7 ps per cell of the batch against 1.2.  Measured on GB300, X-drop 20, both sides of reads in
+// windows, milliseconds of the DP as (pairs, groups): reads of 60, 250 seeds (0.13, 0.15) and 32,000
+// (0.17, 0.89); of 150, 250 (0.83, 0.76), 2,000 (0.85, 0.88), 32,000 (1.12, 4.38); of 300, 1,000
+// (3.07, 1.66), 4,000 (3.10, 2.66), 8,000 (3.11, 3.92), 32,000 (4.16, 11.9).
+bool ext_pairs_fit(const gba_extend_align_params *p, const std::vector<int32_t> &mat, const ExtSides &x)
+{
+    if (!x.valid || x.count < kX2MinSides || x.nmax > kX2Most || x.mmax > kX2MostCols ||
+        x.m.size() >= size_t(1) << 30) return false;
+    const bool affine = p->gap_open != p->gap_extend;
+    if (p->gap_open >= 0 || p->gap_extend > 0 || p->gap_open < -kX2Most || p->gap_extend < -kX2Most) return false;
+    if (!affine && p->gap_extend == 0) return false;
+    int max_pos = 0;
+    if (mat.empty()) {
+        if (std::abs(p->match) > kX2Most || std::abs(p->mismatch) > kX2Most) return false;
+        max_pos = std::max({0, int(p->match), int(p->mismatch)});
+    } else {
+        for (int32_t v : mat) {
+            if (std::abs(v) > kX2Most) return false;
+            max_pos = std::max(max_pos, int(v));
+        }
+    }
+    gba_params gp{};
+    gp.gap_open = p->gap_open;
+    gp.gap_extend = p->gap_extend;
+    if (!w2_fits(gp, max_pos, x.mmax, x.nmax, false)) return false;
+    const double cells = double(x.cells), cols = double(x.mmax), strips = double((x.nmax + kX2Rows - 1) / kX2Rows);
+    const double chunks = 1 + std::floor(0.7 * cells / double(kExtTraceBudget));
+    return 0.46 * cols * strips * chunks + 1.2e-6 * cells <= 4 * cols + 7e-6 * cells;
+}
+
+const void *x2_fn(bool affine, bool matrix)
+{
+    if (affine)
+        return matrix ? reinterpret_cast<const void *>(k_extend2<true, true>) : reinterpret_cast<const void *>(k_extend2<true, false>);
+    return matrix ? reinterpret_cast<const void *>(k_extend2<false, true>) : reinterpret_cast<const void *>(k_extend2<false, false>);
+}
+
+// The extensions of a batch, two per thread; the sequences are in ctx->seq_h and ctx->seq_v.
+int ext_paired(gba_context *ctx, const gba_extend_align_params *p, const std::vector<int32_t> &mat,
+               const gba_seed_batch *b, const gba_seed *seeds, const ExtSides &x, gba_extend_align_result *res)
+{
+    static_assert(sizeof(X2Seed) == sizeof(gba_seed) && sizeof(ExtSegment) == sizeof(gba_segment), "layouts");
+    const int64_t ns = b->num_seeds, ids = 2 * ns;
+    const bool affine = p->gap_open != p->gap_extend, matrix = !mat.empty();
+    cudaStream_t st = ctx->stream;
+    GBA_CUDA(ctx, ctx->xa_seeds.ensure(size_t(ns) * sizeof(gba_seed)));
+    GBA_CUDA(ctx, ctx->xa_off_h.ensure(size_t(b->num_h + 1) * 8));
+    GBA_CUDA(ctx, ctx->xa_off_v.ensure(size_t(b->num_v + 1) * 8));
+    GBA_CUDA(ctx, cudaMemcpyAsync(ctx->xa_seeds.ptr, seeds, size_t(ns) * sizeof(gba_seed), cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(ctx->xa_off_h.ptr, b->off_h, size_t(b->num_h + 1) * 8, cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(ctx->xa_off_v.ptr, b->off_v, size_t(b->num_v + 1) * 8, cudaMemcpyHostToDevice, st));
+    X2Args a{};
+    a.seq_h = ctx->seq_h.as<uint8_t>();
+    a.seq_v = ctx->seq_v.as<uint8_t>();
+    a.off_h = ctx->xa_off_h.as<int64_t>();
+    a.off_v = ctx->xa_off_v.as<int64_t>();
+    a.seeds = ctx->xa_seeds.as<X2Seed>();
+    if (b->seed_h || b->seed_v) {
+        GBA_CUDA(ctx, ctx->xa_ids.ensure(size_t(ns) * 8));
+        int32_t *d = ctx->xa_ids.as<int32_t>();
+        if (b->seed_h) {
+            GBA_CUDA(ctx, cudaMemcpyAsync(d, b->seed_h, size_t(ns) * 4, cudaMemcpyHostToDevice, st));
+            a.seed_h = d;
+        }
+        if (b->seed_v) {
+            GBA_CUDA(ctx, cudaMemcpyAsync(d + ns, b->seed_v, size_t(ns) * 4, cudaMemcpyHostToDevice, st));
+            a.seed_v = d + ns;
+        }
+    }
+    if (matrix) {
+        GBA_CUDA(ctx, ctx->xs_matrix.ensure(mat.size() * 4));
+        GBA_CUDA(ctx, cudaMemcpyAsync(ctx->xs_matrix.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, st));
+        a.matrix = ctx->xs_matrix.as<int32_t>();
+        a.asize = p->alphabet_size;
+    }
+
+    // Sides by strips and columns, the costliest first; neighbours share a thread.  Columns are sorted
+    // to the step that keeps the keys in the sort's one-pass range.
+    const uint32_t strips_max = uint32_t((x.nmax + kX2Rows - 1) / kX2Rows);
+    uint32_t step = 1;
+    while ((uint64_t(x.mmax) / step + 1) * (strips_max + 1) > 16384) step *= 2;
+    const uint32_t span = uint32_t(x.mmax) / step + 1;
+    std::vector<uint32_t> keys(size_t(x.count));
+    std::vector<int32_t> idx(size_t(x.count));
+    for (int64_t id = 0, w = 0; id < ids; ++id)
+        if (x.m[id]) {
+            idx[w] = int32_t(id);
+            keys[w++] = uint32_t((x.n[id] + kX2Rows - 1) / kX2Rows) * span + uint32_t(x.m[id]) / step;
+        }
+    sort_desc(keys, idx);
+    const int64_t nw = (x.count + 63) / 64;
+    std::vector<int32_t> order(size_t(nw) * 64, -1), cols(static_cast<size_t>(nw)), cap(static_cast<size_t>(nw));
+    std::vector<int64_t> tlen(static_cast<size_t>(nw)), toff(static_cast<size_t>(nw)), soff(size_t(nw) + 1, 0);
+#pragma omp parallel for num_threads(plan_threads(x.count)) schedule(static)
+    for (int64_t w = 0; w < nw; ++w) {
+        int32_t mm = 0, nn = 0;
+        for (int64_t q = 0; q < 64 && w * 64 + q < x.count; ++q) {
+            const int32_t id = idx[w * 64 + q];
+            order[w * 64 + (q & 1) * 32 + (q >> 1)] = id;
+            mm = std::max(mm, x.m[id]);
+            nn = std::max(nn, x.n[id]);
+        }
+        cols[w] = mm;
+        cap[w] = mm + nn + 2;
+        tlen[w] = x2_trace_bytes(mm, nn);
+    }
+    std::vector<int64_t> first(1, 0);      // chunks of warps whose trace fits the budget
+    int64_t used = 0, most = 0;
+    for (int64_t w = 0; w < nw; ++w) {
+        if (used && size_t(used + tlen[w]) > kExtTraceBudget) {
+            first.push_back(w);
+            used = 0;
+        }
+        toff[w] = used;
+        used += tlen[w];
+        most = std::max(most, used);
+        soff[w + 1] = soff[w] + 64 * int64_t(cap[w]);
+    }
+    first.push_back(nw);
+
+    const void *fn = x2_fn(affine, matrix);
+    const int64_t grid = std::min<int64_t>(persistent_grid(ctx, fn), (nw + 3) / 4);
+    a.state_rows = int32_t(strips_max * kX2Rows);
+    const size_t order_b = size_t(nw) * 64 * 4, word_b = (size_t(nw) * 4 + 15) & ~size_t(15), long_b = size_t(nw + 1) * 8;
+    GBA_CUDA(ctx, ctx->xa_tasks.ensure(order_b + 2 * word_b + 2 * long_b));
+    uint8_t *pl = ctx->xa_tasks.as<uint8_t>();
+    int32_t *d_order = reinterpret_cast<int32_t *>(pl), *d_cols = reinterpret_cast<int32_t *>(pl + order_b),
+            *d_cap = reinterpret_cast<int32_t *>(pl + order_b + word_b);
+    int64_t *d_toff = reinterpret_cast<int64_t *>(pl + order_b + 2 * word_b),
+            *d_soff = reinterpret_cast<int64_t *>(pl + order_b + 2 * word_b + long_b);
+    GBA_CUDA(ctx, cudaMemcpyAsync(d_order, order.data(), order_b, cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(d_cols, cols.data(), size_t(nw) * 4, cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(d_cap, cap.data(), size_t(nw) * 4, cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(d_toff, toff.data(), size_t(nw) * 8, cudaMemcpyHostToDevice, st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(d_soff, soff.data(), size_t(nw + 1) * 8, cudaMemcpyHostToDevice, st));
+    size_t tmp = 0;
+    GBA_CUDA(ctx, cub::DeviceScan::ExclusiveSum(nullptr, tmp, (int64_t *)nullptr, (int64_t *)nullptr, int(ids + 1), st));
+    GBA_CUDA(ctx, ctx->xa_tmp.ensure(tmp));
+    GBA_CUDA(ctx, ctx->xa_out.ensure(size_t(ids) * sizeof(X2Out)));
+    GBA_CUDA(ctx, ctx->xa_trace.ensure(size_t(most) + 16));
+    GBA_CUDA(ctx, ctx->xa_scratch.ensure(size_t(grid) * 4 * size_t(a.state_rows) * 32 * sizeof(uint2)));
+    GBA_CUDA(ctx, ctx->xa_next.ensure(16));
+    GBA_CUDA(ctx, ctx->xa_segs.ensure(size_t(soff[nw]) * sizeof(ExtSegment)));
+    GBA_CUDA(ctx, ctx->xa_segoff.ensure(size_t(ids) * 8));
+    GBA_CUDA(ctx, ctx->xa_segcnt.ensure(size_t(ids) * 4));
+    GBA_CUDA(ctx, ctx->xa_packoff.ensure(2 * size_t(ids + 1) * 8));
+    GBA_CUDA(ctx, ctx->xa_scores.ensure(size_t(ids) * 4));
+    int32_t *count = ctx->xa_segcnt.as<int32_t>();
+    int64_t *slot = ctx->xa_segoff.as<int64_t>(), *packed_off = ctx->xa_packoff.as<int64_t>(),
+            *wide = packed_off + ids + 1;
+    a.match = p->match;
+    a.mismatch = p->mismatch;
+    a.gap_open = p->gap_open;
+    a.gap_extend = p->gap_extend;
+    a.xdrop_on = p->xdrop_on;
+    a.xdrop = p->xdrop;
+    a.next = ctx->xa_next.as<int32_t>();
+    a.cells = reinterpret_cast<unsigned long long *>(a.next + 2);
+    a.trace = ctx->xa_trace.as<uint8_t>();
+    a.state = ctx->xa_scratch.as<uint2>();
+    a.out = ctx->xa_out.as<X2Out>();
+    GBA_CUDA(ctx, cudaMemsetAsync(a.next, 0, 16, st));
+    GBA_CUDA(ctx, cudaMemsetAsync(count, 0xff, size_t(ids) * 4, st));
+
+    float dp_ms = 0, tb_ms = 0;
+    int launches = 0;
+    for (size_t c = 0; c + 1 < first.size(); ++c) {
+        const int64_t w0 = first[c];
+        X2Args at = a;
+        at.order = d_order + w0 * 64;
+        at.cols = d_cols + w0;
+        at.trace_off = d_toff + w0;
+        at.num_warps = int32_t(first[c + 1] - w0);
+        if (c) GBA_CUDA(ctx, cudaMemsetAsync(a.next, 0, 4, st));
+        GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));
+        void *args[] = {&at};
+        GBA_CUDA(ctx, cudaLaunchKernel(fn, dim3(unsigned(std::min<int64_t>(grid, (at.num_warps + 3) / 4))), dim3(128),
+                                       args, 0, st));
+        GBA_CUDA(ctx, cudaEventRecord(ctx->ev[1], st));
+        const unsigned tg = unsigned((int64_t(at.num_warps) * 64 + 127) / 128);
+        if (affine)
+            k_extend2_traceback<true><<<tg, 128, 0, st>>>(at, d_soff + w0, d_cap + w0, ctx->xa_segs.as<ExtSegment>(), slot, count);
+        else
+            k_extend2_traceback<false><<<tg, 128, 0, st>>>(at, d_soff + w0, d_cap + w0, ctx->xa_segs.as<ExtSegment>(), slot, count);
+        GBA_CUDA(ctx, cudaGetLastError());
+        GBA_CUDA(ctx, cudaEventRecord(ctx->ev[2], st));
+        launches += 2;
+        if (c + 2 < first.size()) {
+            GBA_CUDA(ctx, cudaStreamSynchronize(st));   // the events are used again
+            float ms1 = 0, ms2 = 0;
+            GBA_CUDA(ctx, cudaEventElapsedTime(&ms1, ctx->ev[0], ctx->ev[1]));
+            GBA_CUDA(ctx, cudaEventElapsedTime(&ms2, ctx->ev[1], ctx->ev[2]));
+            dp_ms += ms1;
+            tb_ms += ms2;
+        }
+    }
+    k_extend2_widen<<<unsigned((ids + 256) / 256), 256, 0, st>>>(count, wide, ids);
+    GBA_CUDA(ctx, cudaGetLastError());
+    GBA_CUDA(ctx, cub::DeviceScan::ExclusiveSum(ctx->xa_tmp.ptr, tmp, wide, packed_off, int(ids + 1), st));
+    GBA_CUDA(ctx, cudaMemcpyAsync(res->segment_offsets, packed_off, size_t(ids + 1) * 8, cudaMemcpyDeviceToHost, st));
+    unsigned long long cells = 0;
+    GBA_CUDA(ctx, cudaMemcpyAsync(&cells, a.cells, 8, cudaMemcpyDeviceToHost, st));
+    GBA_CUDA(ctx, cudaStreamSynchronize(st));
+    float ms1 = 0, ms2 = 0;
+    GBA_CUDA(ctx, cudaEventElapsedTime(&ms1, ctx->ev[0], ctx->ev[1]));
+    GBA_CUDA(ctx, cudaEventElapsedTime(&ms2, ctx->ev[1], ctx->ev[2]));
+    const int64_t total = res->segment_offsets[ids];
+    if (total > res->segment_capacity || (total && !res->segments))
+        return fail(ctx, GBA_ECAPACITY, "segment_capacity too small");
+    GBA_CUDA(ctx, ctx->xa_packed.ensure(size_t(std::max<int64_t>(total, 1)) * sizeof(ExtSegment)));
+    int32_t *score = ctx->xa_scores.as<int32_t>();
+    k_extend2_pack<<<unsigned((ids + 127) / 128), 128, 0, st>>>(a, ids, ctx->xa_segs.as<ExtSegment>(), slot, count,
+                                                                packed_off, ctx->xa_packed.as<ExtSegment>(), score,
+                                                                score + ns);
+    GBA_CUDA(ctx, cudaGetLastError());
+    if (total)
+        GBA_CUDA(ctx, cudaMemcpyAsync(res->segments, ctx->xa_packed.ptr, size_t(total) * sizeof(ExtSegment),
+                                      cudaMemcpyDeviceToHost, st));
+    if (res->left_score)
+        GBA_CUDA(ctx, cudaMemcpyAsync(res->left_score, score, size_t(ns) * 4, cudaMemcpyDeviceToHost, st));
+    if (res->right_score)
+        GBA_CUDA(ctx, cudaMemcpyAsync(res->right_score, score + ns, size_t(ns) * 4, cudaMemcpyDeviceToHost, st));
+    GBA_CUDA(ctx, cudaStreamSynchronize(st));
+    ctx->stats = gba_stats{};
+    ctx->stats.dp_kernel_ms = dp_ms + ms1;
+    ctx->stats.traceback_kernel_ms = tb_ms + ms2;
+    ctx->stats.kernel_launches = launches + 3;
+    ctx->stats.cells = int64_t(cells);
+    ctx->stats.tile_rows = kX2Rows;
+    return GBA_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -245,6 +530,15 @@ GBA_API int gba_extend_alignments(gba_context *ctx, const gba_extend_align_param
     if (hb_total) GBA_CUDA(ctx, cudaMemcpyAsync(ctx->seq_h.ptr, b->seq_h, hb_total, cudaMemcpyHostToDevice, st));
     if (vb_total) GBA_CUDA(ctx, cudaMemcpyAsync(ctx->seq_v.ptr, b->seq_v, vb_total, cudaMemcpyHostToDevice, st));
     const uint8_t *dh = ctx->seq_h.as<uint8_t>(), *dv = ctx->seq_v.as<uint8_t>();
+    if (2 * ns >= kX2MinSides) {
+        const ExtSides sides = ext_sides(params, b, seeds);
+        if (ext_pairs_fit(params, mat, sides)) {
+            if (int rc = ext_paired(ctx, params, mat, b, seeds, sides, res)) return rc;
+            ctx->stats.call_ms =
+                std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+            return GBA_OK;
+        }
+    }
 
     // Tasks: (alignment, side) in alignment order; task_of[2k + side] = task index or -1.
     std::vector<ExtTask> tasks;
