@@ -1,12 +1,14 @@
 // enum_host.cuh -- host side of gba_local_enumerate (included at the end of engine.cu).
 //
-// Each pair gets its own scratch in HBM (score matrix, forbidden flags, heap, trace steps and
-// segment slots, about 17 bytes per matrix cell plus the slots); pairs are processed in chunks
-// whose scratch fits kEnumScratchBudget.  After the kernel the per-alignment segment counts come
+// A warp per pair where all pairs fit it (enum_warp_fits), with scratch for the resident warps; otherwise
+// each pair gets its own scratch in HBM (score matrix, forbidden flags, heap and trace steps, about
+// 17 bytes per matrix cell).  Pairs are processed in chunks whose scratch and segment slots fit
+// kEnumScratchBudget.  After the kernel the per-alignment segment counts come
 // back, the host lays out the dense output and a pack kernel copies the used slots.
 #pragma once
 
 #include "enum_kernels.cuh"
+#include "enum_warp_kernels.cuh"
 
 namespace {
 
@@ -34,6 +36,23 @@ int64_t enum_band_cells(int64_t m, int64_t n, int64_t lower, int64_t upper)
     if (m - lower >= 0 && m - lower < hi_fill) hi_fill = m - lower;
     if (m <= 0 || n <= 0 || hi_init - lo_row + 1 <= 0 || hi_fill - lo_row + 1 <= 0) return 0;
     return W * (hi_init - lo_row + 1);
+}
+
+// True when a warp may enumerate an m x n pair (enum_warp_kernels.cuh): values stay from 0 up in 15
+// bits (no match scores below 0, gaps and other pairs never raise a score beyond max_pos per residue
+// pair), positions in 16, the steps of a trace in shared memory.
+bool enum_warp_fits(const gba_enum_params &p, const std::vector<int32_t> &mat, int64_t m, int64_t n)
+{
+    if (p.gap > 0 || m + n > kWeSteps || (m + 1) * (n + 1) > int64_t(1) << kWePosBits) return false;
+    int64_t max_pos = std::max(p.match, p.mismatch);
+    if (mat.empty()) {
+        if (p.match < 0) return false;
+    } else {
+        max_pos = *std::max_element(mat.begin(), mat.end());
+        for (int c = 0; c < p.alphabet_size; ++c)
+            if (mat[size_t(c) * p.alphabet_size + c] < 0) return false;
+    }
+    return max_pos * std::min(m, n) < 32768;
 }
 
 // gba_local_enumerate (band == nullptr) and gba_local_enumerate_banded (band = {lower, upper}).
@@ -83,6 +102,8 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
     std::vector<EnumPair> pairs(static_cast<size_t>(N));
     std::vector<size_t> need(static_cast<size_t>(N));
     std::vector<int64_t> cells_of(static_cast<size_t>(N));
+    // One warp per pair if every pair of the batch fits it, else one thread per pair.
+    bool warps = band == nullptr;
     for (int64_t k = 0; k < N; ++k) {
         const int64_t h0 = b->h_shared ? b->off_h[0] : b->off_h[k], h1 = b->h_shared ? b->off_h[1] : b->off_h[k + 1];
         const int64_t v0 = b->off_v[k], v1 = b->off_v[k + 1];
@@ -106,7 +127,11 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         need[k] = size_t(cells) * 5 + size_t(d.heap_cap) * 8 + size_t(2 * (m + n + 5)) * 4 +
                   size_t(K) * size_t(m + n + 1) * 16 + 64;
         if (need[k] > kEnumScratchBudget) return fail(ctx, GBA_EUNSUPPORTED, "pair %lld needs more scratch than one chunk", (long long)k);
+        warps = warps && enum_warp_fits(*params, mat, m, n);
     }
+    if (warps)
+        for (int64_t k = 0; k < N; ++k)
+            need[k] = size_t(K) * size_t(pairs[k].m + pairs[k].n + 1) * 16 + 64;
     std::vector<int64_t> slot_off(size_t(N) * K, 0);
     int64_t w = 0;   // segments written to the result
     float dp_ms = 0;
@@ -138,10 +163,12 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
             go += int64_t(K) * (d.m + d.n + 1);
         }
         GBA_CUDA(ctx, ctx->en_pairs.ensure(size_t(nc) * sizeof(EnumPair)));
-        GBA_CUDA(ctx, ctx->en_mat.ensure(size_t(mo) * 4 + 16));
-        GBA_CUDA(ctx, ctx->en_forb.ensure(size_t(fo) + 16));
-        GBA_CUDA(ctx, ctx->en_heap.ensure(size_t(ho) * 8 + 16));
-        GBA_CUDA(ctx, ctx->en_steps.ensure(size_t(so) * 4 + 16));
+        if (!warps) {
+            GBA_CUDA(ctx, ctx->en_mat.ensure(size_t(mo) * 4 + 16));
+            GBA_CUDA(ctx, ctx->en_forb.ensure(size_t(fo) + 16));
+            GBA_CUDA(ctx, ctx->en_heap.ensure(size_t(ho) * 8 + 16));
+            GBA_CUDA(ctx, ctx->en_steps.ensure(size_t(so) * 4 + 16));
+        }
         GBA_CUDA(ctx, ctx->en_slots.ensure(size_t(go) * 16 + 16));
         GBA_CUDA(ctx, ctx->en_out.ensure(size_t(na) * 6 * 4 + size_t(nc) * 2 * 4 + 64));
         GBA_CUDA(ctx, cudaMemcpyAsync(ctx->en_pairs.ptr, pairs.data() + c0, size_t(nc) * sizeof(EnumPair),
@@ -177,8 +204,36 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         a.cutoff = params->cutoff;
         a.max_count = K;
         GBA_CUDA(ctx, cudaMemsetAsync(a.seg_count, 0, size_t(na) * 4, st));
-        GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));
-        {
+        if (warps) {
+            int64_t cells = 1, nodes = 1;
+            std::vector<uint32_t> keys(static_cast<size_t>(nc));
+            std::vector<int32_t> order(static_cast<size_t>(nc));
+            for (int64_t k = 0; k < nc; ++k) {
+                keys[k] = uint32_t(cells_of[c0 + k]);
+                order[k] = int32_t(k);
+                cells = std::max(cells, cells_of[c0 + k]);
+                nodes = std::max(nodes, pairs[c0 + k].heap_cap);
+            }
+            sort_desc(keys, order);
+            WeWarpArgs wa{};
+            wa.e = a;
+            wa.mat_at = (nodes + 2) * 4 + 127 & ~int64_t(127);
+            wa.stride = wa.mat_at + cells * 2 + 127 & ~int64_t(127);
+            const size_t smem = kWeWarps * kWeWords * 4;
+            const int64_t grid = std::min(
+                {persistent_grid(ctx, reinterpret_cast<const void *>(&k_waterman_eggert_warp), smem),
+                 (nc + kWeWarps - 1) / kWeWarps, std::max<int64_t>(1, int64_t(kEnumScratchBudget) / (kWeWarps * wa.stride))});
+            GBA_CUDA(ctx, ctx->en_mat.ensure(size_t(grid * kWeWarps * wa.stride)));
+            GBA_CUDA(ctx, ctx->en_steps.ensure(size_t(nc) * 4));
+            GBA_CUDA(ctx, cudaMemcpyAsync(ctx->en_steps.ptr, order.data(), size_t(nc) * 4, cudaMemcpyHostToDevice, st));
+            wa.scratch = ctx->en_mat.as<uint8_t>();
+            wa.order = ctx->en_steps.as<int32_t>();
+            wa.next = o + 6 * na + 2 * nc;
+            GBA_CUDA(ctx, cudaMemsetAsync(wa.next, 0, 4, st));
+            GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));
+            k_waterman_eggert_warp<<<unsigned(grid), 32 * kWeWarps, smem, st>>>(wa);
+        } else {
+            GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));
             // Each pair is one thread's sequential enumeration whose heap and declump steps take
             // data-dependent branches, so the lanes of a warp diverge and run one after another.
             // A warp therefore takes few pairs -- the smallest power of two that still fits
@@ -190,11 +245,11 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
             const int64_t resident = persistent_grid(ctx, fn) * (kBlock / 32);
             a.lanes = 2;
             while (a.lanes < 32 && 2 * int64_t(a.lanes) * resident < nc) a.lanes *= 2;
-            const int64_t warps = (nc + a.lanes - 1) / a.lanes;
+            const int64_t blocks = (nc + a.lanes - 1) / a.lanes;
             if (band)
-                k_waterman_eggert_banded<<<unsigned(warps), 32, 0, st>>>(a, band[0], band[1]);
+                k_waterman_eggert_banded<<<unsigned(blocks), 32, 0, st>>>(a, band[0], band[1]);
             else
-                k_waterman_eggert<<<unsigned(warps), 32, 0, st>>>(a);
+                k_waterman_eggert<<<unsigned(blocks), 32, 0, st>>>(a);
         }
         GBA_CUDA(ctx, cudaGetLastError());
         GBA_CUDA(ctx, cudaEventRecord(ctx->ev[1], st));

@@ -10,7 +10,8 @@
 // scores go where the reference's heap puts them, so the heap's push / pop / adjust-top steps are
 // the reference's.
 //
-// One thread per pair: an enumeration is sequential (each alignment depends on the declumped
+// Here one thread per pair (enum_warp_kernels.cuh takes batches of unbanded pairs of up to 2^16 cells, a
+// warp per pair): an enumeration is sequential (each alignment depends on the declumped
 // matrix of the previous one, and the heap's tie order on the exact sequence of pushes), so the
 // batch's pairs run in parallel.  Each pair's scratch -- the (m+1) x (n+1) score matrix, the
 // forbidden flags, the heap (at most m * n entries) and the trace steps -- sits in HBM at offsets
