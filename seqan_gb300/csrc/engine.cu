@@ -861,53 +861,71 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     // groups of 64, thread l of a warp holding slots l and 32 + l.  The other pairs follow, one a thread.
     plan->duo_slots = 0;
     if (band2_ok && !idx.empty()) {
+        const int64_t count = int64_t(idx.size());
         int64_t fit = 0;
         int32_t m0 = INT32_MAX, m1 = 0, n0 = INT32_MAX, n1 = 0;
-        for (int32_t k : idx)
-            if (desc[k].rows) {
-                ++fit;
-                m0 = std::min(m0, desc[k].m);
-                m1 = std::max(m1, desc[k].m);
-                n0 = std::min(n0, desc[k].n);
-                n1 = std::max(n1, desc[k].n);
-            }
+#pragma omp parallel for num_threads(plan_threads(count)) schedule(static) reduction(+ : fit) \
+    reduction(min : m0, n0) reduction(max : m1, n1)
+        for (int64_t i = 0; i < count; ++i) {
+            const PairDesc &d = desc[idx[i]];
+            if (!d.rows) continue;
+            ++fit;
+            m0 = std::min(m0, d.m);
+            m1 = std::max(m1, d.m);
+            n0 = std::min(n0, d.n);
+            n1 = std::max(n1, d.n);
+        }
+        const bool one_size = fit > 0 && m0 == m1 && n0 == n1;
         std::vector<int32_t> duo, rest;
-        duo.reserve(size_t(fit));
-        rest.reserve(idx.size() - size_t(fit) + 64);
-        for (int32_t k : idx) (desc[k].rows ? duo : rest).push_back(k);
-        if (m0 < m1 || n0 < n1) {
+        if (fit == count) {
+            duo.swap(idx);
+        } else {
+            duo.reserve(size_t(fit));
+            rest.reserve(size_t(count - fit) + 64);
+            for (int32_t k : idx) (desc[k].rows ? duo : rest).push_back(k);
+        }
+        std::vector<uint32_t> dk;
+        if (!one_size) {
             const uint32_t span = uint32_t(n1 - n0 + 1);
-            std::vector<uint32_t> dk(duo.size());
-            for (size_t i = 0; i < duo.size(); ++i) dk[i] = uint32_t(desc[duo[i]].m - m0) * span + uint32_t(desc[duo[i]].n - n0);
+            dk.resize(duo.size());
+#pragma omp parallel for num_threads(plan_threads(fit)) schedule(static)
+            for (int64_t i = 0; i < fit; ++i)
+                dk[i] = uint32_t(desc[duo[i]].m - m0) * span + uint32_t(desc[duo[i]].n - n0);
             sort_desc(dk, duo);
         }
-        auto same = [&](int32_t x, int32_t y) { return desc[x].m == desc[y].m && desc[x].n == desc[y].n; };
-        // neighbours of one size make a duo; an odd one out goes with the rest
-        std::vector<int32_t> lo, hi;
-        lo.reserve(duo.size() / 2 + 32);
-        hi.reserve(duo.size() / 2 + 32);
-        for (size_t i = 0; i < duo.size();) {
-            if (i + 1 < duo.size() && same(duo[i], duo[i + 1])) {
-                lo.push_back(duo[i]);
-                hi.push_back(duo[i + 1]);
-                i += 2;
-            } else {
-                desc[duo[i]].rows = 0;
-                rest.push_back(duo[i++]);
+        // neighbours of one size make a duo (at duo[first[q]], or duo[2 q] where all are); an odd one out
+        // goes with the rest
+        std::vector<int32_t> first;
+        int64_t duos = 0;
+        auto odd_out = [&](int32_t k) {
+            desc[k].rows = 0;
+            rest.push_back(k);
+        };
+        if (one_size) {
+            duos = fit / 2;
+            if (fit & 1) odd_out(duo[fit - 1]);
+        } else {
+            first.reserve(size_t(fit / 2));
+            for (int64_t i = 0; i < fit;) {
+                if (i + 1 < fit && dk[i] == dk[i + 1]) {
+                    first.push_back(int32_t(i));
+                    i += 2;
+                } else {
+                    odd_out(duo[i++]);
+                }
             }
+            duos = int64_t(first.size());
         }
-        lo.resize((lo.size() + 31) / 32 * 32, -1);
-        hi.resize(lo.size(), -1);
-        plan->duo_slots = int64_t(lo.size()) * 2;
+        plan->duo_slots = (duos + 31) / 32 * 64;
         idx.resize(size_t(plan->duo_slots) + rest.size());
 #pragma omp parallel for num_threads(plan_threads(plan->duo_slots)) schedule(static)
-        for (int64_t q = 0; q < int64_t(lo.size()); ++q) {
-            const int64_t at = q / 32 * 64 + q % 32;
-            idx[at] = lo[q];
-            idx[at + 32] = hi[q];
-            if (lo[q] >= 0) {
-                desc[lo[q]].rows = 1;      // low half
-                desc[hi[q]].rows = 2;      // high half
+        for (int64_t q = 0; q < plan->duo_slots / 2; ++q) {
+            const int64_t at = q / 32 * 64 + q % 32, i = q >= duos ? -1 : (one_size ? 2 * q : first[q]);
+            idx[at] = i < 0 ? -1 : duo[i];
+            idx[at + 32] = i < 0 ? -1 : duo[i + 1];
+            if (i >= 0) {
+                desc[duo[i]].rows = 1;         // low half
+                desc[duo[i + 1]].rows = 2;     // high half
             }
         }
         std::copy(rest.begin(), rest.end(), idx.begin() + plan->duo_slots);
