@@ -589,16 +589,16 @@ OPS_PER_CELL = {"affine_global": 9, "linear_global": 5, "affine_local": 10, "lin
 CAPTURED = {
     "affine_dna_100k": {"dram_bytes_per_cell": (143.7e6 + 361.7e6) / 4.336e9, "alu_pipe_pct": 80.8,
                         "profile": "profiles/k_dp16x2_affine_dna_100k.md"},
-    "banded_reads_1m": {"dram_bytes_per_cell": (367.6e6 + 837.0e6) / 9.816e8, "alu_pipe_pct": 57.5,
+    "banded_reads_1m": {"dram_bytes_per_cell": (1171.0e6 + 3802.3e6) / 4.908e9, "alu_pipe_pct": 74.6,
                         "profile": "profiles/k_dp_banded_reads_1m.md"},
-    "protein_local_tb_20k": {"dram_bytes_per_cell": (13.5e6 + 626.4e6) / 9.732e8, "alu_pipe_pct": 78.9,
+    "protein_local_tb_20k": {"dram_bytes_per_cell": (48.8e6 + 2689.3e6) / 2.41e9, "alu_pipe_pct": 80.8,
                              "profile": "profiles/k_dp_warp2_protein_local_tb.md"},
 }
 
 KERNEL_NAMES = [(2, "k_pack16 + k_dp16x2 (two pairs per thread, DPX int16x2)"),
-                (16, "k_dp_warp2 (64 strips per warp in int16x2 halves, 4-bit trace)"),
+                (16, "k_dp_warp2 (64 strips of 2-8 rows per warp in int16x2 halves, 4-bit trace)"),
                 (4, "k_dp_warp (one warp per 256-row band, anti-diagonal front)"),
-                (8, "k_dp_banded (one pair per thread, band in per-thread slots)"),
+                (8, "k_dp_banded2 / k_dp_banded (two pairs of equal lengths, or one, per thread)"),
                 (1, "k_dp_strip (one pair per thread, int32)"),
                 (32, "k_dp_dynamic (DynamicGaps cells, one pair per thread, int32)")]
 
@@ -1219,14 +1219,15 @@ def run_extend_bench(args, rank, world, local_rank, dist):
     peak = C.c_double()
     ctx.check(L.gba_measure_int_peak(h, C.byref(peak)), "int peak")
     dp_ms = sum(dpk) / len(dpk)
-    ops = 2 * st.cells * OPS_PER_CELL["affine_global"]     # score pass + trace pass over the same cells
+    passes = 1 if st.tile_rows == 16 else 2                # k_extend_dp: a score pass and a trace pass
+    ops = passes * st.cells * OPS_PER_CELL["affine_global"]
     achieved = ops / (dp_ms * 1e-3) / 1e12
     line = {"metric": "M alignments/s, batched extendAlignment (X-drop)", "value": value, "unit": "M alignments/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": kernel_ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
             "config": {"workload": args.workload, "description": WORKLOADS[args.workload], "alignments": n_al,
                        "cells_per_step": int(st.cells), "rows_per_band": int(st.tile_rows),
-                       "value_timing": "CUDA events around the score pass, trace pass and traceback inside "
+                       "value_timing": "CUDA events around the DP and the traceback inside "
                                        "gba_extend_alignments (inputs in HBM)",
                        "parallelism": f"replicas x{world}"},
             "e2e": {"value": e2e, "unit": "M alignments/s",
@@ -1236,9 +1237,10 @@ def run_extend_bench(args, rank, world, local_rank, dist):
             "gpu_launches": args.steps * int(st.kernel_launches),
             "roofline": {"bound": "int32", "achieved": achieved, "peak": peak.value, "unit": "Tops/s",
                          "frac": achieved / peak.value if peak.value else None, "traffic": None,
-                         "kernel": "k_extend_dp<affine> (score and trace passes) + k_extend_traceback",
+                         "kernel": "k_extend2<affine> + k_extend2_traceback" if st.tile_rows == 16 else
+                                   "k_extend_dp<affine> (score and trace passes) + k_extend_traceback",
                          "ops_per_cell": OPS_PER_CELL["affine_global"], "dp_kernel_ms": dp_ms,
-                         "gcups_per_pass": st.cells / (dp_ms / 2 * 1e-3) / 1e9,
+                         "gcups_per_pass": st.cells / (dp_ms / passes * 1e-3) / 1e9,
                          "peak_source": "measured live by gba_measure_int_peak (32-bit add+max issue rate)"},
             "clocks": clocks, "parity_first_2000_vs_oracle": parity}
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
@@ -1376,7 +1378,9 @@ def run_we_bench(args, rank, world, local_rank, dist):
     # the initial fill alone: linear local, 6 ops per cell (two gap adds, diagonal add, two maxima,
     # the zero floor); the heap, the traces and the declumping come on top
     achieved = cells * OPS_PER_CELL["linear_local"] / (kernel_ms * 1e-3) / 1e12
-    kname = "k_waterman_eggert_banded" if band else "k_waterman_eggert"
+    kname = ("k_waterman_eggert_banded (one thread per pair: heap, traces and declumping are sequential per pair)"
+             if band else "k_waterman_eggert_warp (one warp per pair: each heap, trace and declumping step across "
+                          "its lanes)")
     line = {"metric": we_metric(band), "value": value,
             "unit": "pairs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": kernel_ms,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
@@ -1391,8 +1395,7 @@ def run_we_bench(args, rank, world, local_rank, dist):
             "gpu_launches": args.steps * int(st.kernel_launches),
             "roofline": {"bound": "latency", "achieved": achieved, "peak": peak.value, "unit": "Tops/s",
                          "frac": achieved / peak.value if peak.value else None, "traffic": None,
-                         "kernel": kname + " (one thread per pair: heap, traces and declumping are sequential "
-                                           "per pair) + k_enum_pack",
+                         "kernel": kname + " + k_enum_pack",
                          "ops_per_cell": OPS_PER_CELL["linear_local"], "dp_kernel_ms": kernel_ms,
                          "note": "achieved counts the initial matrix fill only" +
                                  (" (the band's cells inside the matrix)" if band else ""),
@@ -1531,7 +1534,7 @@ def run_chain_bench(args, rank, world, local_rank, dist):
             "gpu_launches": args.steps * int(st.kernel_launches),
             "roofline": {"bound": "latency", "achieved": achieved, "peak": peak.value, "unit": "Tops/s",
                          "frac": achieved / peak.value if peak.value else None, "traffic": None,
-                         "kernel": "k_banded_chain (one thread per chain: its grids, tracebacks and glue in order) "
+                         "kernel": "k_banded_chain (one warp per chain: its grids, tracebacks and glue in order) "
                                    "+ k_chain_pack",
                          "ops_per_cell": OPS_PER_CELL["affine_global"], "dp_kernel_ms": kernel_ms,
                          "peak_source": "measured live by gba_measure_int_peak (32-bit add+max issue rate)"},

@@ -125,8 +125,9 @@ typedef struct {
  * int16 range and the batch holds at least 32768 pairs.  Other unbanded pairs whose values fit 16
  * bits (gap scores from -1024 to 0, every score between about -31,600 and 32,700) run the packed
  * 16-bit warp kernel (two strips per lane; equality scoring needs alphabet_size 1..8 there too), with
- * 16- and 32-bit score types alike; the remaining unbanded pairs run the 32-bit warp kernel, banded
- * pairs one thread per pair. */
+ * 16- and 32-bit score types alike; the remaining unbanded pairs run the 32-bit warp kernel.
+ * Banded pairs run one per thread, or two per thread where both have the same lengths and values of
+ * 16 bits (bands of up to 40 diagonals). */
 enum {
     GBA_FLAG_GENERAL_KERNEL = 1,   /* force the one-pair-per-thread 32-bit kernel */
     GBA_FLAG_STRIP16 = 2,          /* packed kernel with 16-row strips instead of 32 */
