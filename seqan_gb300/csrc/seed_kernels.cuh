@@ -185,7 +185,14 @@ __global__ void __launch_bounds__(kSeedBlock) k_extend_simple(SeedArgs a)
 
 template <int RING> struct XMinBlocks { static constexpr int value = RING <= 16 ? 5 : (RING <= 32 ? 3 : 2); };
 
-constexpr int kRefillLanes = 8;   // idle lanes that trigger a warp refill
+template <int RING> struct XMask { using type = uint32_t; };
+template <> struct XMask<64> { using type = uint64_t; };
+__device__ __forceinline__ int low_bit(uint32_t x) { return __ffs(int(x)) - 1; }
+__device__ __forceinline__ int low_bit(uint64_t x) { return __ffsll((long long)x) - 1; }
+__device__ __forceinline__ int high_bit(uint32_t x) { return 31 - __clz(int(x)); }
+__device__ __forceinline__ int high_bit(uint64_t x) { return 63 - __clzll((long long)x); }
+
+constexpr int kRefillLanes = 4;   // idle lanes that trigger a warp refill (8: +1.3%, 14: +6%)
 
 // Rings per thread, one word per slot: anti-diagonals k-2, k-1, k, then the query residues by
 // column and the database residues by row.  Both residue windows only slide forward: per
@@ -232,6 +239,8 @@ __global__ void __launch_bounds__(kSeedBlock, STRIDE == 1 ? 4 : XMinBlocks<RING>
     int lo1 = 0, hi1 = 0, lo2 = 0, hi2 = 0, lo3 = 0, hi3 = 0;
     int qnext = 0, dnext = 0;             // next column / row whose residue is not loaded yet
     int qpend = -1, dpend = -1;           // residues loaded at the previous step, stored at this one
+    using Mask = typename XMask<RING>::type;
+    Mask defined = 0;                     // the last anti-diagonal's defined cells, bit 0 at lo3
     uint64_t cells = 0;
 #define XR(r, c) (r)[((c) & rmask) * STRIDE]
 #define XB(r, c) XR(r, c)
@@ -259,6 +268,7 @@ __global__ void __launch_bounds__(kSeedBlock, STRIDE == 1 ? 4 : XMinBlocks<RING>
         const int g0 = (-gap > xdrop) ? U : gap;
         base[(2 * ring) * STRIDE] = g0;
         base[(2 * ring + 1) * STRIDE] = g0;
+        defined = g0 != U ? 3 : 0;
         minCol = 1;
         maxCol = 2;
         k = 1;
@@ -403,24 +413,60 @@ __global__ void __launch_bounds__(kSeedBlock, STRIDE == 1 ? 4 : XMinBlocks<RING>
         int up = XR(r2, lo3);
         // The reference's minCol / maxCol scans (:708-721) read back what this loop writes: the
         // first column c >= minCol with A3[c] or A2[c-1] defined, and the last column
-        // c >= minCol - 1 with A3[c] or A2[c] defined.  Both are tracked here instead.
-        int lastLive = (blo != U || up != U) ? lo3 : lo3 - 1;
-        int firstLive = INT_MAX;
+        // c >= minCol - 1 with A3[c] or A2[c] defined.
+        int firstLive, lastLive;
+        if (STRIDE != 1) {
+            // Rings in shared memory: which cells of an anti-diagonal are defined fits a word (bit
+            // c - lo), so a cell only adds its bit; ring offsets step instead of being masked anew.
+            // Bound by issue (1M read seeds, X = 20: 5.24 ms with both tracked cell by cell, as below,
+            // 4.73 so; unrolled 1, 3 and 4 times 4.98, 4.95 and 4.90).  With a ring, thr = best - X stays
+            // far above `undefined`, so a cell >= thr is defined.
+            constexpr int kWrap = RING * STRIDE - 1;
+            const Mask before = defined >> (lo3 - lo2);                  // A2, by column from lo3
+            Mask now = 0, bit = 2;
+            int o = (minCol & rmask) * STRIDE, left = (lo3 & rmask) * STRIDE, od = ((k - minCol) & rmask) * STRIDE;
 #pragma unroll 2
-        for (int col = minCol; col < maxCol; ++col) {
-            const int cur = XR(r2, col);
-            const int dg = XR(r1, col - 1);
-            const int sub = sc(XB(qres, col), XB(dres, k - col));
-            int t = max(max(up, cur) + gap, dg + sub);
-            const bool def = t >= thr;
-            t = def ? t : U;
-            XR(r3, col) = t;
-            dbest = max(dbest, t);    // `undefined` never exceeds k * gap
-            firstLive = min(firstLive, (def || up != U) ? col : INT_MAX);
-            lastLive = (def || cur != U) ? col : lastLive;
-            up = cur;
+            for (int col = minCol; col < maxCol; ++col) {
+                const int cur = r2[o];
+                const int sub = sc(qres[o], dres[od]);
+                int t = max(max(up, cur) + gap, r1[left] + sub);
+                const bool def = t >= thr;
+                t = def ? t : U;
+                r3[o] = t;
+                dbest = max(dbest, t);    // `undefined` never exceeds k * gap
+                now |= def ? bit : Mask(0);
+                bit += bit;
+                up = cur;
+                left = o;
+                o = (o + STRIDE) & kWrap;
+                od = (od - STRIDE) & kWrap;
+            }
+            const int width = maxCol - lo3;                              // (1 .. RING - 1)
+            const Mask inside = (Mask(1) << width) - 1;
+            const Mask first = (now | before << 1) & inside & ~Mask(1);
+            const Mask last = ((now | before) & inside) | Mask(blo != U ? 1 : 0);
+            const bool end = bhi != U || (before >> (width - 1) & 1);
+            firstLive = first ? lo3 + low_bit(first) : (end ? maxCol : maxCol + 1);
+            lastLive = last ? lo3 + high_bit(last) : lo3 - 1;
+            defined = now | Mask(blo != U ? 1 : 0) | Mask(bhi != U ? 1 : 0) << (hi3 - lo3);
+        } else {
+            lastLive = (blo != U || up != U) ? lo3 : lo3 - 1;
+            firstLive = INT_MAX;
+            for (int col = minCol; col < maxCol; ++col) {
+                const int cur = XR(r2, col);
+                const int dg = XR(r1, col - 1);
+                const int sub = sc(XB(qres, col), XB(dres, k - col));
+                int t = max(max(up, cur) + gap, dg + sub);
+                const bool def = t >= thr;
+                t = def ? t : U;
+                XR(r3, col) = t;
+                dbest = max(dbest, t);
+                firstLive = min(firstLive, (def || up != U) ? col : INT_MAX);
+                lastLive = (def || cur != U) ? col : lastLive;
+                up = cur;
+            }
+            if (firstLive == INT_MAX) firstLive = (bhi != U || up != U) ? maxCol : maxCol + 1;
         }
-        if (firstLive == INT_MAX) firstLive = (bhi != U || up != U) ? maxCol : maxCol + 1;
         best = max(best, dbest);
         minCol = firstLive;
         maxCol = lastLive + 2;
