@@ -210,6 +210,7 @@ int ext_banded(gba_context *ctx, const gba_extend_align_params *params, const st
 constexpr int64_t kX2MinSides = 512;
 constexpr int kX2Most = 1024;                    // scores and gap costs, and rows of a side
 constexpr int kX2MostCols = 4096;
+constexpr size_t kX2SlotBudget = size_t(16) << 30;
 
 // The sides of a batch: their number, sizes and cells.
 struct ExtSides {
@@ -256,7 +257,9 @@ ExtSides ext_sides(const gba_extend_align_params *p, const gba_seed_batch *b, co
 }
 
 // True when two sides per thread is the form for a batch: gaps cost something (the best cell then
-// never ends in one), values fit 16 bits, and the time expected is the shorter.  A thread takes
+// never ends in one), values fit 16 bits, the segment slots of all sides (sized by the largest of their
+// warp; the groups size them by the columns computed) stay within kX2SlotBudget, and the time expected is
+// the shorter.  A thread takes
 // 0.46 us per column of a strip and has the whole side to itself; trace chunks follow one another.
 // A group of lanes takes 4 us per column (both passes), so it is done first with a few sides, but
 // costs 7 ps per cell of the batch against 1.2.  Measured on GB300, X-drop 20, both sides of reads in
@@ -284,6 +287,7 @@ bool ext_pairs_fit(const gba_extend_align_params *p, const std::vector<int32_t> 
     gp.gap_open = p->gap_open;
     gp.gap_extend = p->gap_extend;
     if (!w2_fits(gp, max_pos, x.mmax, x.nmax, false)) return false;
+    if (size_t(x.count + 64) * size_t(x.mmax + x.nmax + 2) * sizeof(ExtSegment) > kX2SlotBudget) return false;
     const double cells = double(x.cells), cols = double(x.mmax), strips = double((x.nmax + kX2Rows - 1) / kX2Rows);
     const double chunks = 1 + std::floor(0.7 * cells / double(kExtTraceBudget));
     return 0.46 * cols * strips * chunks + 1.2e-6 * cells <= 4 * cols + 7e-6 * cells;
