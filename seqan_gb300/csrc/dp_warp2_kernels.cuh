@@ -447,7 +447,10 @@ struct W2Input {
         nextCode = H[min(c0 + (lane & (kW2Chunk - 1)), m - 1)];
     }
     // Makes the chunk at c0 (loaded before) the current one, waiting until its entries are there,
-    // and loads the next.  Columns past m get values of no effect.
+    // and loads the next.  Lanes past column m keep the row above that they have: a strip's low half runs
+    // 32 columns ahead of its high one, so it is past m while the high half holds real cells, and beside
+    // a value from elsewhere (a zero, say) a cell with a score near the range's ends could differ from
+    // its neighbours by more than 2^15, which w2_equal would carry into the high half.
     __device__ __forceinline__ void advance(int c0, int32_t *error)
     {
         const int c = c0 + (lane & (kW2Chunk - 1));
@@ -465,7 +468,8 @@ struct W2Input {
                     load_row(c0);
                 }
             }
-            above = c <= m ? uint32_t(next) : w2_pack(0, kW2Inf);
+            if (c <= m) above = uint32_t(next);
+            if (c0 == 0 && m < kW2Chunk - 1) above = __shfl_sync(0xffffffffu, uint32_t(next), min(lane, m));
         } else {
             above = w2_pack(w2_row0(c, fTop, affine, open, ext), kW2Inf);
         }
