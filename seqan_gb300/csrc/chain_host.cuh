@@ -77,7 +77,6 @@ GBA_API int gba_banded_chain(gba_context *ctx, const gba_chain_params *params, c
         pl.gseg_cap = d.m + d.n + 8;
         chain::Engine e{};
         e.plan = true;
-        e.warp = false;
         e.anchor = anchor;
         e.gap = gap;
         e.fe = params->free_ends;

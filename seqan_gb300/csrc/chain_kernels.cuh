@@ -150,7 +150,6 @@ __host__ __device__ inline int mxc(int &target, int left, int right, int tl, int
 struct Engine {
     // ---- configuration ----
     bool plan;                  // plan mode: geometry only
-    bool warp;                  // one warp per chain: grids filled by anti-diagonals across the lanes
     Scheme anchor, gap;
     int fe, affine, k;
     int max_traces;
@@ -185,9 +184,27 @@ struct Engine {
     Cell bestCell;
 
     __host__ __device__ void fail(int code) { if (!err) err = code; }
+    // On the device all lanes of a warp run the driver on one engine.  Lane 0 alone changes its state and
+    // the chain's scratch, between enter() and leave(): the other lanes have read what they need before
+    // the first barrier and see the changes behind the second, so that all take the same way.  What the
+    // lanes do together (clearing, the fill of a grid) writes disjoint places and ends in a barrier.
 #ifdef __CUDA_ARCH__
     static __device__ __forceinline__ int lane_id() { return int(threadIdx.x & 31); }
+    static __device__ __forceinline__ int lane_count() { return 32; }
+    static __device__ __forceinline__ bool enter() { __syncwarp(); return lane_id() == 0; }
+    static __device__ __forceinline__ void leave() { __syncwarp(); }
+#else
+    static __host__ int lane_id() { return 0; }
+    static __host__ int lane_count() { return 1; }
+    static __host__ bool enter() { return true; }
+    static __host__ void leave() {}
 #endif
+    // fail() by all lanes
+    __host__ __device__ void fail_all(int code)
+    {
+        if (enter()) fail(code);
+        leave();
+    }
 
     // =========================== init-cell set ===========================
     GBA_CHAIN_STEP __host__ __device__ bool set_insert(int i1, int i2, Cell c)
@@ -210,44 +227,34 @@ struct Engine {
         return true;
     }
 
-    // _reinitScoutState
+    // _reinitScoutState, and an empty local trace set
     GBA_CHAIN_STEP __host__ __device__ void reinit(int64_t oh, int64_t ov, int64_t ch, int64_t cv, int64_t nh, int64_t nv)
     {
         if (err) return;
         const int64_t want[4] = {ch, cv, nh, nv};
-        if (oh < 0 || ov < 0 || ch < 0 || cv < 0 || nh < 0 || nv < 0) { fail(ST_UNDEFINED); return; }
-        if (ch > (1 << 30) || cv > (1 << 30) || nh > (1 << 30) || nv > (1 << 30)) { fail(ST_UNDEFINED); return; }
-        hNext = oh;
-        vNext = ov;
-        for (int q = 0; q < 4; ++q) {
-            if (n4[q] < want[q]) n4[q] = int(want[q]);
-            if (plan) {
-                if (pl->vlen[q] < n4[q]) pl->vlen[q] = n4[q];
-                continue;
+        if (oh < 0 || ov < 0 || ch < 0 || cv < 0 || nh < 0 || nv < 0) { fail_all(ST_UNDEFINED); return; }
+        if (ch > (1 << 30) || cv > (1 << 30) || nh > (1 << 30) || nv > (1 << 30)) { fail_all(ST_UNDEFINED); return; }
+        if (enter()) {
+            hNext = oh;
+            vNext = ov;
+            nl = 0;
+            for (int q = 0; q < 4; ++q) {
+                if (n4[q] < want[q]) n4[q] = int(want[q]);
+                if (plan && pl->vlen[q] < n4[q]) pl->vlen[q] = n4[q];
             }
-#ifdef __CUDA_ARCH__
-            if (warp) {
-                for (int i = lane_id(); i < n4[q]; i += 32) w.v4[q][i] = Cell{INF, INF, INF};
-                continue;
-            }
-#endif
-            for (int i = 0; i < n4[q]; ++i) w.v4[q][i] = Cell{INF, INF, INF};
         }
-#ifdef __CUDA_ARCH__
-        if (warp) __syncwarp();
-#endif
+        leave();
         if (plan) return;
-        for (int i = 0; i < nset; ++i) {
-            const InitCell &e = w.set[i];
-            if (e.i1 == 0) {
-                if (e.i2 >= n4[1]) { fail(ST_UNDEFINED); return; }
-                w.v4[1][e.i2] = e.c;
+        for (int q = 0; q < 4; ++q)
+            for (int i = lane_id(); i < n4[q]; i += lane_count()) w.v4[q][i] = Cell{INF, INF, INF};
+        if (enter())
+            for (int i = 0; i < nset; ++i) {
+                const InitCell &e = w.set[i];
+                if ((e.i1 == 0 && e.i2 >= n4[1]) || (e.i2 == 0 && e.i1 >= n4[0])) { fail(ST_UNDEFINED); break; }
+                if (e.i1 == 0) w.v4[1][e.i2] = e.c;
+                if (e.i2 == 0) w.v4[0][e.i1] = e.c;
             }
-            if (e.i2 == 0) {
-                if (e.i1 >= n4[0]) { fail(ST_UNDEFINED); return; }
-                w.v4[0][e.i1] = e.c;
-            }
-        }
+        leave();
     }
 
     // =========================== traces ===========================
@@ -328,6 +335,11 @@ struct Engine {
     GBA_CHAIN_STEP __host__ __device__ void glue_local(int64_t gbh, int64_t gbv, bool check_empty)
     {
         if (plan || err) return;
+        if (enter()) glue(gbh, gbv, check_empty);
+        leave();
+    }
+    __host__ __device__ void glue(int64_t gbh, int64_t gbv, bool check_empty)
+    {
         for (int i = 0; i < nl; ++i) {
             Seg *ls = lslot(i);
             for (int q = 0; q < w.llen[i]; ++q) {
@@ -337,12 +349,7 @@ struct Engine {
         }
         if (check_empty && nl == 0) return;
         if (ng == 0) {
-            for (int i = 0; i < nl; ++i) {
-                const int g = new_global();
-                if (g < 0) return;
-                g_prepend(g, lslot(i), w.llen[i]);
-            }
-            nl = 0;
+            take_local();
             return;
         }
         const int n0 = ng;
@@ -395,14 +402,31 @@ struct Engine {
     __host__ __device__ void assign_global_from_local()
     {
         if (plan || err) return;
-        ng = 0;
-        gused = 0;
+        if (enter()) {
+            ng = 0;
+            gused = 0;
+            take_local();
+        }
+        leave();
+    }
+    // the local traces become the last global ones
+    __host__ __device__ void take_local()
+    {
         for (int i = 0; i < nl; ++i) {
             const int g = new_global();
             if (g < 0) return;
             g_prepend(g, lslot(i), w.llen[i]);
         }
         nl = 0;
+    }
+    // the next grid begins this much further on
+    __host__ __device__ void advance(int64_t dh, int64_t dv)
+    {
+        if (enter()) {
+            hNext += dh;
+            vNext += dv;
+        }
+        leave();
     }
 
     // =========================== grid DP ===========================
@@ -962,15 +986,49 @@ struct Engine {
     {
         if (err) return INT_MIN;
         if (pm <= 0 || pn <= 0) return INT_MIN;
-        if (pm > (1 << 28) || pn > (1 << 28)) { fail(ST_UNDEFINED); return INT_MIN; }
+        if (pm > (1 << 28) || pn > (1 << 28)) { fail_all(ST_UNDEFINED); return INT_MIN; }
         if (bd) {
             if (up < -pn || lw > pm) return INT_MIN;
             if (up < 0 && !(fe & FREE_LEFT)) return INT_MIN;
             if (lw > 0 && !(fe & FREE_TOP)) return INT_MIN;
             if (up + pn < pm && !(fe & FREE_BOTTOM)) return INT_MIN;
             if (lw + pn > pm && !(fe & FREE_RIGHT)) return INT_MIN;
-            if (up == lw) { fail(ST_UNDEFINED); return INT_MIN; }
+            if (up == lw) { fail_all(ST_UNDEFINED); return INT_MIN; }
         }
+        if (enter()) set_grid(s, kd, bd, lw, up, ph, pm, pv, pn);
+        leave();
+        if (err) return INT_MIN;
+        if (plan) return 0;
+#ifdef __CUDA_ARCH__
+        for (int64_t q = lane_id(); q < (L * Hlen + 15) / 16; q += 32) reinterpret_cast<uint4 *>(w.T)[q] = make_uint4(0, 0, 0, 0);
+#endif
+        if (kd != KIND_GLOBAL) {
+            leave();
+            fill_warp();
+        } else {
+            if (enter()) {
+                if (bd) run_banded();
+                else run_unbanded();
+            }
+            leave();
+        }
+        if (err) return INT_MIN;
+        if (enter()) {
+            if (kd == KIND_GLOBAL) {
+                global_trace();
+            } else {
+                nset = 0;
+                for (int i = 0; i < nmp && !err; ++i) chain_trace_one(w.mp[i]);
+            }
+        }
+        leave();
+        return kd == KIND_GLOBAL ? bestS : maxS;
+    }
+
+    // The grid's sizes, its navigator's start and an empty scout; plan mode: the chain's maxima.
+    __host__ __device__ void set_grid(const Scheme *s, int kd, bool bd, int lw, int up, const uint8_t *ph, int64_t pm,
+                                      const uint8_t *pv, int64_t pn)
+    {
         sc = s; kind = kd; banded = bd; lower = lw; upper = up;
         gh = ph; gv = pv; gm = int(pm); gn = int(pn);
         if (bd) {
@@ -986,7 +1044,7 @@ struct Engine {
             leap = 1;
             pos = 0;
         }
-        if (L * Hlen >= (int64_t(1) << 31)) { fail(ST_CAPACITY); return INT_MIN; }   // positions are 32-bit
+        if (L * Hlen >= (int64_t(1) << 31)) { fail(ST_CAPACITY); return; }   // positions are 32-bit
         if (plan) {
             if (bd) {
                 for (int64_t j = 0; j <= pm; ++j) {
@@ -1003,18 +1061,11 @@ struct Engine {
             if (pl->mp_cap < mpb) pl->mp_cap = int32_t(mpb);
             if (pl->lseg_cap < pm + pn + 8) pl->lseg_cap = int32_t(pm + pn + 8);
             if (pl->col_cap < pm + 1) pl->col_cap = int32_t(pm + 1);
-            return 0;
+            return;
         }
-        if (L * Hlen > pl->trace_bytes || pn + 1 > pl->col_rows) { fail(ST_CAPACITY); return INT_MIN; }
-#ifdef __CUDA_ARCH__
+        if (L * Hlen > pl->trace_bytes || pn + 1 > pl->col_rows) { fail(ST_CAPACITY); return; }
         w.T = L * Hlen <= kSharedTrace ? w.sharedT : w.arenaT;
         w.cols = pm + 1 <= kSharedCols ? w.sharedCols : w.arenaCols;
-        __syncwarp();
-        for (int64_t q = lane_id(); q < (L * Hlen + 15) / 16; q += 32) reinterpret_cast<uint4 *>(w.T)[q] = make_uint4(0, 0, 0, 0);
-        __syncwarp();
-#else
-        for (int64_t q = 0; q < L * Hlen; ++q) w.T[q] = 0;
-#endif
         lo0 = lo1 = INT_MAX;
         hi0 = hi1 = -1;
         maxS = INF;
@@ -1022,17 +1073,6 @@ struct Engine {
         bestS = INF;
         bestPos = 0;
         bestCol = bestRow = 0;
-        if (warp && kd != KIND_GLOBAL) fill_warp();
-        else if (bd) run_banded();
-        else run_unbanded();
-        if (err) return INT_MIN;
-        if (kd == KIND_GLOBAL) {
-            global_trace();
-            return bestS;
-        }
-        nset = 0;
-        for (int i = 0; i < nmp && !err; ++i) chain_trace_one(w.mp[i]);
-        return maxS;
     }
 
     // ---------------- warp-cooperative fill ----------------
@@ -1330,17 +1370,16 @@ struct Engine {
         const int lane = lane_id();
         const bool mine = p_ >= 0 && s_ == maxS;
         const unsigned who = __ballot_sync(0xffffffffu, mine);
-        if (nmp + __popc(who) > pl->mp_cap) { fail(ST_CAPACITY); return; }
-        if (mine) w.mp[nmp + __popc(who & ((1u << lane) - 1u))] = p_;
-        const int n = nmp + __popc(who);
-        __syncwarp();
-        nmp = n;
-        __syncwarp();
+        const int at = nmp, n = at + __popc(who);
+        if (n > pl->mp_cap) { fail_all(ST_CAPACITY); return; }
+        if (mine) w.mp[at + __popc(who & ((1u << lane) - 1u))] = p_;
+        if (enter()) nmp = n;
+        leave();
     }
 
     __device__ void fill_warp()
     {
-        if (gm + 1 > pl->col_cap || gn + 1 > pl->col_rows) { fail(ST_CAPACITY); return; }
+        if (gm + 1 > pl->col_cap || gn + 1 > pl->col_rows) { fail_all(ST_CAPACITY); return; }
         const int lane = lane_id();
         for (int r = lane; r <= gn; r += 32) w.fcP[r] = -1;
         int cfirst = 0, clast = 0;
@@ -1381,9 +1420,8 @@ struct Engine {
             if (w.fcP[r] >= 0) best = cmax(best, w.fcS[r]);
         best = __reduce_max_sync(0xffffffffu, best);
         if (best < maxS) return;
-        __syncwarp();
-        maxS = best;
-        __syncwarp();
+        if (enter()) maxS = best;
+        leave();
         for (int c0 = cfirst; c0 <= clast && !err; c0 += 32) {
             const int c = c0 + lane;
             collect(c <= clast ? w.cols[c].candS : 0, c <= clast ? w.cols[c].candP : -1);
@@ -1407,6 +1445,11 @@ struct Engine {
     __host__ __device__ static int64_t vse(const Seed &s) { return s.up - s.eh + s.ev; }
 
     __host__ __device__ void init_beginning(int64_t sizeH, int64_t sizeV, const Scheme &s)
+    {
+        if (enter()) set_beginning(sizeH, sizeV, s);
+        leave();
+    }
+    __host__ __device__ void set_beginning(int64_t sizeH, int64_t sizeV, const Scheme &s)
     {
         Cell c{0, INF, INF};
         set_insert(0, 0, c);
@@ -1436,16 +1479,11 @@ struct Engine {
         if (hN != 0 || vN != 0) {
             init_beginning(up + 1, 1 - lw, gap);
             reinit(hN, vN, 1 + up, 1 - lw, 1 + up - hN, 1 - lw - vN);
-            nl = 0;
             score = run_grid(&gap, KIND_INITIAL, false, 0, 0, h, up, v, -lw);
             // the initial gap area writes into the global set directly
             if (!plan && !err) {
-                for (int i = 0; i < nl; ++i) {
-                    const int g = new_global();
-                    if (g < 0) break;
-                    g_prepend(g, lslot(i), w.llen[i]);
-                }
-                nl = 0;
+                if (enter()) take_local();
+                leave();
             }
         } else {
             init_beginning(up, -lw, anchor);
@@ -1459,8 +1497,7 @@ struct Engine {
         lw += gbv;
         if (lv + lw > up) vN2 -= (lv + lw) - up;
         reinit(hN2, vN2, up + 1, 1 - lw, lh - hN2 + 1, lv - vN2 + 1);
-        if (lh < 0 || lv < 0) { fail(ST_UNDEFINED); return INT_MIN; }
-        nl = 0;
+        if (lh < 0 || lv < 0) { fail_all(ST_UNDEFINED); return INT_MIN; }
         if (gbh == 0 && gbv == 0) {
             if (geh == m && gev == n) score = run_grid(&gap, KIND_GLOBAL, true, int(lw), int(up), h, lh, v, lv);
             else score = run_grid(&gap, KIND_INITIAL, true, int(lw), int(up), h, lh, v, lv);
@@ -1470,9 +1507,7 @@ struct Engine {
         }
         if (gbh != 0 || gbv != 0) glue_local(gbh, gbv, true);
         else assign_global_from_local();
-        hNext += gbh;
-        vNext += gbv;
-        if (lv + lw > up) vNext += (lv + lw) - up;
+        advance(gbh, gbv + (lv + lw > up ? (lv + lw) - up : 0));
         return score;
     }
 
@@ -1481,13 +1516,11 @@ struct Engine {
         const int64_t gbh = hNext, gbv = vNext;
         const int64_t geh = s.bh + 1 + k + hsb(s), gev = s.bv + 1 + k + vsb(s);
         const int64_t hN = s.bh + 1 - k - gbh, vN = s.bv + 1 - k - gbv;
-        if (geh > m || gev > n || gbh > geh || gbv > gev) { fail(ST_UNDEFINED); return; }
+        if (geh > m || gev > n || gbh > geh || gbv > gev) { fail_all(ST_UNDEFINED); return; }
         reinit(hN, vN, geh - gbh + 1, gev - gbv + 1, geh - gbh + 1 - hN, gev - gbv + 1 - vN);
-        nl = 0;
         run_grid(&gap, KIND_INNER, false, 0, 0, h + gbh, geh - gbh, v + gbv, gev - gbv);
         glue_local(gbh, gbv, true);
-        hNext += gbh;
-        vNext += gbv;
+        advance(gbh, gbv);
     }
 
     __host__ __device__ void anchor_area(const Seed &s)
@@ -1498,15 +1531,12 @@ struct Engine {
         const int64_t hN = s.eh - k - hse(s) - gbh, vN = s.ev - k - vse(s) - gbv;
         const int64_t lw = -2 * k - vsb(s), up = 2 * k + hsb(s);
         int64_t relV = vN;
-        if (geh > m || gev > n || lh < 0 || lv < 0) { fail(ST_UNDEFINED); return; }
+        if (geh > m || gev > n || lh < 0 || lv < 0) { fail_all(ST_UNDEFINED); return; }
         if (lv + lw > up) relV -= (lv + lw) - up;
         reinit(hN, relV, up + 1, 1 - lw, lh - hN + 1, lv - vN + 1);
-        nl = 0;
         run_grid(&anchor, KIND_INNER, true, int(lw), int(up), h + gbh, lh, v + gbv, lv);
         glue_local(gbh, gbv, true);
-        hNext += gbh;
-        vNext += gbv;
-        if (lv + lw > up) vNext += (lv + lw) - up;
+        advance(gbh, gbv + (lv + lw > up ? (lv + lw) - up : 0));
     }
 
     __host__ __device__ int finish(const Seed &s)
@@ -1517,9 +1547,8 @@ struct Engine {
         int64_t lh = geh - gbh, lv = gev - gbv;
         int64_t hN = cmax<int64_t>(0, s.bh + 1 - k - gbh), vN = cmax<int64_t>(0, s.bv + 1 - k - gbv);
         int score;
-        if (lh < 0 || lv < 0) { fail(ST_UNDEFINED); return INT_MIN; }
+        if (lh < 0 || lv < 0) { fail_all(ST_UNDEFINED); return INT_MIN; }
         reinit(hN, vN, lh + 1, lv + 1, lh - hN + 1, lv - vN + 1);
-        nl = 0;
         run_grid(&gap, KIND_INNER, false, 0, 0, h + gbh, lh, v + gbv, lv);
         glue_local(gbh, gbv, true);
         gbh += hN;
@@ -1528,11 +1557,10 @@ struct Engine {
         gev = cmin<int64_t>(n, s.ev + k);
         lh = geh - gbh;
         lv = gev - gbv;
-        if (lh < 0 || lv < 0) { fail(ST_UNDEFINED); return INT_MIN; }
+        if (lh < 0 || lv < 0) { fail_all(ST_UNDEFINED); return INT_MIN; }
         if (geh == m && gev == n) {
             const int64_t lw = -(gev - gbv), up = geh - gbh;
             reinit(0, 0, up + 1, 1 - lw, up + 1, 1 - lw);
-            nl = 0;
             score = run_grid(&anchor, KIND_FINAL, true, int(lw), int(up), h + gbh, lh, v + gbv, lv);
             glue_local(gbh, gbv, true);
             return score;
@@ -1542,15 +1570,13 @@ struct Engine {
         vN = cmax<int64_t>(0, s.ev - k - vse(s) - gbv - cmax<int64_t>(0, s.eh + k - m));
         if (lv + lw > up) vN -= (lv + lw) - up;
         reinit(hN, vN, up + 1, 1 - lw, lh - hN + 1, lv - vN + 1);
-        nl = 0;
         run_grid(&anchor, KIND_INNER, true, int(lw), int(up), h + gbh, lh, v + gbv, lv);
         glue_local(gbh, gbv, true);
         gbh += hN;
         if (lv + lw > up) vN += (lv + lw) - up;
         gbv += vN;
-        if (gbh > m || gbv > n) { fail(ST_UNDEFINED); return INT_MIN; }
+        if (gbh > m || gbv > n) { fail_all(ST_UNDEFINED); return INT_MIN; }
         reinit(0, 0, m - gbh + 1, n - gbv + 1, m - gbh + 1, n - gbv + 1);
-        nl = 0;
         score = run_grid(&gap, KIND_FINAL, false, 0, 0, h + gbh, m - gbh, v + gbv, n - gbv);
         glue_local(gbh, gbv, true);
         return score;
@@ -1559,15 +1585,18 @@ struct Engine {
     // The whole chain; returns the score (status in err).
     __host__ __device__ int run(const int32_t *seeds, int ns)
     {
-        err = 0;
-        hNext = vNext = 0;
-        n4[0] = n4[1] = n4[2] = n4[3] = 0;
-        nset = 0;
-        ng = 0;
-        gused = 0;
-        nl = 0;
+        if (enter()) {
+            err = 0;
+            hNext = vNext = 0;
+            n4[0] = n4[1] = n4[2] = n4[3] = 0;
+            nset = 0;
+            ng = 0;
+            gused = 0;
+            nl = 0;
+        }
+        leave();
         if (ns < 1) return INT_MIN;
-        if (m <= 0 || n <= 0 || k < 1) { fail(ST_UNDEFINED); return INT_MIN; }
+        if (m <= 0 || n <= 0 || k < 1) { fail_all(ST_UNDEFINED); return INT_MIN; }
         auto seed = [&](int i) {
             Seed s;
             s.bh = seeds[4 * i]; s.bv = seeds[4 * i + 1]; s.eh = seeds[4 * i + 2]; s.ev = seeds[4 * i + 3];
@@ -1597,7 +1626,6 @@ struct Engine {
             if (s.eh + k < m || s.ev + k < n) {
                 const int64_t gbh = hNext, gbv = vNext;
                 reinit(0, 0, m + 1 - gbh, n + 1 - gbv, m + 1 - gbh, n + 1 - gbv);
-                nl = 0;
                 score = run_grid(&gap, KIND_FINAL, false, 0, 0, h + gbh, m - gbh, v + gbv, n - gbv);
                 glue_local(gbh, gbv, false);
             }
@@ -1614,9 +1642,8 @@ struct Engine {
     }
 };
 
-// A warp's part of the block's shared memory.  The engine is one per warp: its lanes run the driver,
-// the tracebacks and the glue in lockstep on the same values (every lane writes what the others
-// write), and 32 private copies of its state overflowed L1.
+// A warp's part of the block's shared memory.  The engine is one per warp (32 private copies of its
+// state overflowed L1): all lanes run the driver, lane 0 changes the state (Engine::enter).
 struct WarpShared {
     uint8_t T[kSharedTrace];
     ColDesc cols[kSharedCols];
@@ -1699,29 +1726,29 @@ __global__ void __launch_bounds__(128, 4) k_banded_chain(ChainArgs a)
         c = __shfl_sync(0xffffffffu, c, 0);
         if (c >= a.num_chains) return;
         const chain::ChainDesc &d = a.chains[c];
-        ws.plan = d.plan;
-        e.plan = false;
-        e.warp = true;
-        e.anchor = a.anchor;
-        e.gap = a.gap;
-        e.fe = a.free_ends;
-        e.affine = a.affine;
-        e.k = a.band_ext;
-        e.max_traces = a.max_traces;
-        e.h = a.seq_h + d.h_off;
-        e.v = a.seq_v + d.v_off;
-        e.m = d.m;
-        e.n = d.n;
-        e.pl = &ws.plan;
-        e.ng = 0;
-        chain::layout(ws.plan, a.max_traces, a.arena + d.arena_off, &e.w);
-        e.w.sharedT = ws.T;
-        e.w.sharedCols = ws.cols;
-        const int status = ws.plan.status;
+        if (lane == 0) {
+            ws.plan = d.plan;
+            e.plan = false;
+            e.anchor = a.anchor;
+            e.gap = a.gap;
+            e.fe = a.free_ends;
+            e.affine = a.affine;
+            e.k = a.band_ext;
+            e.max_traces = a.max_traces;
+            e.h = a.seq_h + d.h_off;
+            e.v = a.seq_v + d.v_off;
+            e.m = d.m;
+            e.n = d.n;
+            e.pl = &ws.plan;
+            e.ng = 0;
+            e.err = d.plan.status;
+            chain::layout(d.plan, a.max_traces, a.arena + d.arena_off, &e.w);
+            e.w.sharedT = ws.T;
+            e.w.sharedCols = ws.cols;
+        }
         __syncwarp();
         int score = INT_MIN;
-        if (status == chain::ST_OK) score = e.run(a.seeds + 4 * d.seed_off, d.n_seeds);
-        else e.err = status;
+        if (d.plan.status == chain::ST_OK) score = e.run(a.seeds + 4 * d.seed_off, d.n_seeds);
         __syncwarp();
         if (lane == 0) {
             a.score[d.id] = score;
