@@ -47,6 +47,7 @@ struct SrvRequest {
     std::vector<uint8_t> h, v;
     double t_submit = 0;
     int64_t bytes = 0;   // device bytes it adds to a batch
+    bool narrow = false; // counted, and to be run, without the packed warp kernel
 };
 
 struct SrvDone {
@@ -88,22 +89,27 @@ struct gba_server {
 
 namespace {
 
-// Device bytes one pair adds to a batch: inputs, per-pair records, row buffers, trace and
-// segment slots (the terms build_plan allocates for it).
-int64_t request_bytes(const gba_params &p, int64_t m, int64_t n)
+// Device bytes one pair adds to a batch: inputs, per-pair records, row buffers, band states, tasks, trace
+// and segment slots (the terms build_plan allocates for it).  narrow: on the 32-bit warp kernel; else on
+// whichever warp kernel takes more, in any of the packed one's rows per strip (two rows make the most
+// bands, of 128 rows).
+int64_t request_bytes(const gba_params &p, int64_t m, int64_t n, bool narrow)
 {
     int64_t b = m + n + int64_t(sizeof(PairDesc)) + 128;
     if (p.outputs & GBA_OUT_SEGMENTS) {
         if (p.band_on) b += (m + 1) * band_col_bytes(p.band_upper - p.band_lower + 1) / 32;
         else {
             int64_t t = warp_trace_bytes(int(m), int(n), kWarpRows);
-            for (int R : {2, 3, 4, 5, 6, 8})
-                t = std::max(t, w2_trace_bytes(int(m), int(n), R, p.mode == GBA_LOCAL));
+            if (!narrow)
+                for (int R : {2, 3, 4, 5, 6, 8})
+                    t = std::max(t, w2_trace_bytes(int(m), int(n), R, p.mode == GBA_LOCAL));
             b += t;
         }
         b += (m + n + 4) * 16 * 2;
     }
-    if (!p.band_on && n > 32 * kWarpRows) b += 2 * (m + 1) * 8 + ((n + 255) / 256) * int64_t(sizeof(BandState));
+    const int64_t band_rows = narrow ? 32 * kWarpRows : 128;
+    if (!p.band_on && n > band_rows)
+        b += 2 * (m + 1) * 8 + ((n + band_rows - 1) / band_rows) * int64_t(sizeof(BandState) + (narrow ? 0 : sizeof(int2)));
     return b;
 }
 
@@ -152,7 +158,10 @@ int srv_launch(gba_server *s, SrvSlot &sl)
     b.off_h = sl.off_h.data();
     b.seq_v = sl.seq_v.as<uint8_t>();
     b.off_v = sl.off_v.data();
-    int rc = build_plan(ctx, &s->params, &b, &sl.plan);
+    gba_params params = s->params;
+    for (const SrvRequest &q : sl.reqs)
+        if (q.narrow) params.flags |= GBA_FLAG_NO_WARP16;
+    int rc = build_plan(ctx, &params, &b, &sl.plan);
     if (rc) return rc;
     GBA_CUDA(ctx, sl.dseq_h.ensure(size_t(sl.plan.seq_h_bytes) + 16));
     GBA_CUDA(ctx, sl.dseq_v.ensure(size_t(sl.plan.seq_v_bytes) + 16));
@@ -364,7 +373,11 @@ GBA_API int gba_server_submit(gba_server *s, uint64_t tag, const uint8_t *h, int
     if (m > (1 << 30) || n > (1 << 30)) return GBA_EINVAL;
     SrvRequest q;
     q.tag = tag;
-    q.bytes = request_bytes(s->params, m, n);
+    q.bytes = request_bytes(s->params, m, n, false);
+    if (s->budget > 0 && q.bytes > s->budget) {
+        q.narrow = true;   // a request that fits the budget on the 32-bit kernel alone runs there
+        q.bytes = request_bytes(s->params, m, n, true);
+    }
     if (s->budget > 0 && q.bytes > s->budget) {
         std::lock_guard<std::mutex> lk(s->mu);
         s->last_error = "request needs " + std::to_string(q.bytes) + " device bytes, budget is " +
