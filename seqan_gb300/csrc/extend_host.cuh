@@ -300,7 +300,8 @@ const void *x2_fn(bool affine, bool matrix)
     return matrix ? reinterpret_cast<const void *>(k_extend2<false, true>) : reinterpret_cast<const void *>(k_extend2<false, false>);
 }
 
-// The extensions of a batch, two per thread; the sequences are in ctx->seq_h and ctx->seq_v.
+// The extensions of a batch, two per thread; the sequences are in ctx->seq_h and ctx->seq_v.  GBA_ENOMEM:
+// there is not enough memory for this form; nothing is promised to the caller yet.
 int ext_paired(gba_context *ctx, const gba_extend_align_params *p, const std::vector<int32_t> &mat,
                const gba_seed_batch *b, const gba_seed *seeds, const ExtSides &x, gba_extend_align_result *res)
 {
@@ -387,6 +388,11 @@ int ext_paired(gba_context *ctx, const gba_extend_align_params *p, const std::ve
     const int64_t grid = std::min<int64_t>(persistent_grid(ctx, fn), (nw + 3) / 4);
     a.state_rows = int32_t(strips_max * kX2Rows);
     const size_t order_b = size_t(nw) * 64 * 4, word_b = (size_t(nw) * 4 + 15) & ~size_t(15), long_b = size_t(nw + 1) * 8;
+    const size_t state_b = size_t(grid) * 4 * size_t(a.state_rows) * 32 * sizeof(uint2);
+    // Under a budget that the trace, the slots and the states exceed, the groups' form runs (its slots are
+    // those of the columns computed), as where the device has not got the memory.
+    if (ctx->budget > 0 && size_t(most) + size_t(soff[nw]) * sizeof(ExtSegment) + state_b > size_t(ctx->budget))
+        return GBA_ENOMEM;
     GBA_CUDA(ctx, ctx->xa_tasks.ensure(order_b + 2 * word_b + 2 * long_b));
     uint8_t *pl = ctx->xa_tasks.as<uint8_t>();
     int32_t *d_order = reinterpret_cast<int32_t *>(pl), *d_cols = reinterpret_cast<int32_t *>(pl + order_b),
@@ -403,7 +409,7 @@ int ext_paired(gba_context *ctx, const gba_extend_align_params *p, const std::ve
     GBA_CUDA(ctx, ctx->xa_tmp.ensure(tmp));
     GBA_CUDA(ctx, ctx->xa_out.ensure(size_t(ids) * sizeof(X2Out)));
     GBA_CUDA(ctx, ctx->xa_trace.ensure(size_t(most) + 16));
-    GBA_CUDA(ctx, ctx->xa_scratch.ensure(size_t(grid) * 4 * size_t(a.state_rows) * 32 * sizeof(uint2)));
+    GBA_CUDA(ctx, ctx->xa_scratch.ensure(state_b));
     GBA_CUDA(ctx, ctx->xa_next.ensure(16));
     GBA_CUDA(ctx, ctx->xa_segs.ensure(size_t(soff[nw]) * sizeof(ExtSegment)));
     GBA_CUDA(ctx, ctx->xa_segoff.ensure(size_t(ids) * 8));
@@ -537,10 +543,19 @@ GBA_API int gba_extend_alignments(gba_context *ctx, const gba_extend_align_param
     if (2 * ns >= kX2MinSides) {
         const ExtSides sides = ext_sides(params, b, seeds);
         if (ext_pairs_fit(params, mat, sides)) {
-            if (int rc = ext_paired(ctx, params, mat, b, seeds, sides, res)) return rc;
-            ctx->stats.call_ms =
-                std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
-            return GBA_OK;
+            const int rc = ext_paired(ctx, params, mat, b, seeds, sides, res);
+            if (rc != GBA_ENOMEM) {
+                ctx->stats.call_ms =
+                    std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
+                return rc;
+            }
+            // What this form did get is given back, and the groups' form takes the batch.
+            GBA_CUDA(ctx, cudaStreamSynchronize(st));
+            for (DevBuf *d : {&ctx->xa_tasks, &ctx->xa_out, &ctx->xa_trace, &ctx->xa_segs, &ctx->xa_segoff, &ctx->xa_segcnt,
+                              &ctx->xa_scratch, &ctx->xa_packoff, &ctx->xa_packed, &ctx->xa_seeds, &ctx->xa_off_h,
+                              &ctx->xa_off_v, &ctx->xa_ids, &ctx->xa_tmp, &ctx->xa_scores})
+                d->release();
+            cudaGetLastError();   // (the failed allocation's)
         }
     }
 
