@@ -13,6 +13,10 @@
 namespace {
 
 constexpr size_t kEnumScratchBudget = size_t(6) << 30;
+// Batches of pairs of at most this many cells run a thread per pair (100,000 pairs of 6 x 6, one
+// alignment: 0.07 ms, a warp per pair 0.13; of 10 x 10 0.20 and 0.19, of 14 x 14 0.39 and 0.27).
+constexpr int64_t kEnumWarpCells = 128;
+constexpr int64_t kEnumUnsorted = 1024;
 
 __global__ void __launch_bounds__(128) k_enum_pack(const uint32_t *slots, const int64_t *slot_off,
                                                    const int32_t *count, const int64_t *dense_off, uint32_t *dense,
@@ -38,21 +42,22 @@ int64_t enum_band_cells(int64_t m, int64_t n, int64_t lower, int64_t upper)
     return W * (hi_init - lo_row + 1);
 }
 
-// True when a warp may enumerate an m x n pair (enum_warp_kernels.cuh): values stay from 0 up in 15
-// bits (no match scores below 0, gaps and other pairs never raise a score beyond max_pos per residue
-// pair), positions in 16, the steps of a trace in shared memory.
-bool enum_warp_fits(const gba_enum_params &p, const std::vector<int32_t> &mat, int64_t m, int64_t n)
+// What a residue pair scores at most where a warp may enumerate pairs of a scheme (no match scores below
+// 0, gaps and other pairs never raise a score beyond it), else -1.
+int64_t enum_warp_scheme(const gba_enum_params &p, const std::vector<int32_t> &mat)
 {
-    if (p.gap > 0 || m + n > kWeSteps || (m + 1) * (n + 1) > int64_t(1) << kWePosBits) return false;
-    int64_t max_pos = std::max(p.match, p.mismatch);
-    if (mat.empty()) {
-        if (p.match < 0) return false;
-    } else {
-        max_pos = *std::max_element(mat.begin(), mat.end());
-        for (int c = 0; c < p.alphabet_size; ++c)
-            if (mat[size_t(c) * p.alphabet_size + c] < 0) return false;
-    }
-    return max_pos * std::min(m, n) < 32768;
+    if (p.gap > 0) return -1;
+    if (mat.empty()) return p.match < 0 ? -1 : std::max(p.match, p.mismatch);
+    for (int c = 0; c < p.alphabet_size; ++c)
+        if (mat[size_t(c) * p.alphabet_size + c] < 0) return -1;
+    return *std::max_element(mat.begin(), mat.end());
+}
+
+// True when a warp may enumerate an m x n pair of such a scheme (enum_warp_kernels.cuh): values stay from 0
+// up in 15 bits, positions in 16, the steps of a trace in shared memory.
+bool enum_warp_fits(int64_t max_pos, int64_t m, int64_t n)
+{
+    return m + n <= kWeSteps && (m + 1) * (n + 1) <= int64_t(1) << kWePosBits && max_pos * std::min(m, n) < 32768;
 }
 
 // gba_local_enumerate (band == nullptr) and gba_local_enumerate_banded (band = {lower, upper}).
@@ -100,10 +105,12 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         GBA_CUDA(ctx, cudaMemcpyAsync(ctx->xs_matrix.ptr, mat.data(), mat.size() * 4, cudaMemcpyHostToDevice, st));
     }
     std::vector<EnumPair> pairs(static_cast<size_t>(N));
-    std::vector<size_t> need(static_cast<size_t>(N));
+    std::vector<size_t> need(static_cast<size_t>(N)), slots(static_cast<size_t>(N));   // of all; of the segments alone
     std::vector<int64_t> cells_of(static_cast<size_t>(N));
     // One warp per pair if every pair of the batch fits it, else one thread per pair.
-    bool warps = band == nullptr;
+    const int64_t max_pos = band ? -1 : enum_warp_scheme(*params, mat);
+    bool warps = max_pos >= 0;
+    int64_t most = 0;
     for (int64_t k = 0; k < N; ++k) {
         const int64_t h0 = b->h_shared ? b->off_h[0] : b->off_h[k], h1 = b->h_shared ? b->off_h[1] : b->off_h[k + 1];
         const int64_t v0 = b->off_v[k], v1 = b->off_v[k + 1];
@@ -124,14 +131,14 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         // cell, and a pair that needs more (max_count > 16) is rerun with the bound
         d.heap_cap = band ? int64_t(K < 16 ? K : 16) * cells + 16 : m * n;
         cells_of[k] = cells;
-        need[k] = size_t(cells) * 5 + size_t(d.heap_cap) * 8 + size_t(2 * (m + n + 5)) * 4 +
-                  size_t(K) * size_t(m + n + 1) * 16 + 64;
+        slots[k] = size_t(K) * size_t(m + n + 1) * 16 + 64;
+        need[k] = size_t(cells) * 5 + size_t(d.heap_cap) * 8 + size_t(2 * (m + n + 5)) * 4 + slots[k];
         if (need[k] > kEnumScratchBudget) return fail(ctx, GBA_EUNSUPPORTED, "pair %lld needs more scratch than one chunk", (long long)k);
-        warps = warps && enum_warp_fits(*params, mat, m, n);
+        warps = warps && enum_warp_fits(max_pos, m, n);
+        most = std::max(most, cells);
     }
-    if (warps)
-        for (int64_t k = 0; k < N; ++k)
-            need[k] = size_t(K) * size_t(pairs[k].m + pairs[k].n + 1) * 16 + 64;
+    warps = warps && most > kEnumWarpCells;
+    if (warps) need.swap(slots);
     std::vector<int64_t> slot_off(size_t(N) * K, 0);
     int64_t w = 0;   // segments written to the result
     float dp_ms = 0;
@@ -146,7 +153,7 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         int32_t *o = nullptr;
         std::vector<int32_t> outh(size_t(na) * 6 + size_t(nc) * 2);
         for (int attempt = 0;; ++attempt) {
-        int64_t mo = 0, fo = 0, ho = 0, so = 0, go = 0;
+        int64_t mo = 0, fo = 0, ho = 0, so = 0, go = 0, nodes = 1;
         for (int64_t k = c0; k < c1; ++k) {
             EnumPair &d = pairs[k];
             const int64_t cells = cells_of[k];
@@ -156,6 +163,7 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
             fo += cells;
             d.heap_off = ho;
             ho += d.heap_cap;
+            nodes = std::max(nodes, d.heap_cap);
             d.step_off = so;
             so += 2 * int64_t(d.m + d.n + 5);
             d.seg_off = go;
@@ -205,29 +213,30 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
         a.max_count = K;
         GBA_CUDA(ctx, cudaMemsetAsync(a.seg_count, 0, size_t(na) * 4, st));
         if (warps) {
-            int64_t cells = 1, nodes = 1;
-            std::vector<uint32_t> keys(static_cast<size_t>(nc));
-            std::vector<int32_t> order(static_cast<size_t>(nc));
-            for (int64_t k = 0; k < nc; ++k) {
-                keys[k] = uint32_t(cells_of[c0 + k]);
-                order[k] = int32_t(k);
-                cells = std::max(cells, cells_of[c0 + k]);
-                nodes = std::max(nodes, pairs[c0 + k].heap_cap);
-            }
-            sort_desc(keys, order);
             WeWarpArgs wa{};
             wa.e = a;
+            // The largest pairs first: one taken last would leave the device to itself.  Pairs of at most
+            // kEnumUnsorted cells take less than 0.1 ms, so that their order costs more than it gives.
+            if (most > kEnumUnsorted) {
+                std::vector<uint32_t> keys(static_cast<size_t>(nc));
+                std::vector<int32_t> order(static_cast<size_t>(nc));
+                for (int64_t k = 0; k < nc; ++k) {
+                    keys[k] = uint32_t(cells_of[c0 + k]);
+                    order[k] = int32_t(k);
+                }
+                sort_desc(keys, order);
+                GBA_CUDA(ctx, ctx->en_steps.ensure(size_t(nc) * 4));
+                GBA_CUDA(ctx, cudaMemcpyAsync(ctx->en_steps.ptr, order.data(), size_t(nc) * 4, cudaMemcpyHostToDevice, st));
+                wa.order = ctx->en_steps.as<int32_t>();
+            }
             wa.mat_at = (nodes + 2) * 4 + 127 & ~int64_t(127);
-            wa.stride = wa.mat_at + cells * 2 + 127 & ~int64_t(127);
+            wa.stride = wa.mat_at + most * 2 + 127 & ~int64_t(127);
             const size_t smem = kWeWarps * kWeWords * 4;
             const int64_t grid = std::min(
                 {persistent_grid(ctx, reinterpret_cast<const void *>(&k_waterman_eggert_warp), smem),
                  (nc + kWeWarps - 1) / kWeWarps, std::max<int64_t>(1, int64_t(kEnumScratchBudget) / (kWeWarps * wa.stride))});
             GBA_CUDA(ctx, ctx->en_mat.ensure(size_t(grid * kWeWarps * wa.stride)));
-            GBA_CUDA(ctx, ctx->en_steps.ensure(size_t(nc) * 4));
-            GBA_CUDA(ctx, cudaMemcpyAsync(ctx->en_steps.ptr, order.data(), size_t(nc) * 4, cudaMemcpyHostToDevice, st));
             wa.scratch = ctx->en_mat.as<uint8_t>();
-            wa.order = ctx->en_steps.as<int32_t>();
             wa.next = o + 6 * na + 2 * nc;
             GBA_CUDA(ctx, cudaMemsetAsync(wa.next, 0, 4, st));
             GBA_CUDA(ctx, cudaEventRecord(ctx->ev[0], st));

@@ -39,7 +39,7 @@ constexpr int kWeWarps = 4;              // warps of a block
 
 struct WeWarpArgs {
     EnumArgs e;                       // mat, forb, heap and steps unused
-    const int32_t *order;             // pairs, the largest first
+    const int32_t *order;             // pairs, the largest first (null: as they come)
     // Per resident warp: heap of m * n + 2 nodes (1-based), then the matrix of (m + 1) * (n + 1) cells
     // (value, bit 15 forbidden), for the largest of the pairs.
     uint8_t *scratch;
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(32 * kWeWarps, 8) k_waterman_eggert_warp(WeWar
         if (w.lane == 0) p = atomicAdd(a.next, 1);
         p = __shfl_sync(0xffffffffu, p, 0);
         if (p >= a.e.num_pairs) return;
-        p = a.order[p];
+        if (a.order) p = a.order[p];
         const EnumPair d = a.e.pairs[p];
         w.H = a.e.seq_h + d.h_off;
         w.V = a.e.seq_v + d.v_off;
