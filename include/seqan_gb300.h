@@ -251,9 +251,13 @@ enum {
     GBA_KERNEL_STRIP = 1,      /* one pair per thread, 16-row register strips, int32 */
     GBA_KERNEL_PACKED = 2,     /* two pairs per thread, int16x2 DPX */
     GBA_KERNEL_WARP = 4,       /* bands of 256 rows, one warp per band, anti-diagonal front */
-    GBA_KERNEL_BANDED = 8,     /* banded DP, one pair per thread */
+    GBA_KERNEL_BANDED = 8,     /* banded DP, one pair per thread; with GBA_KERNEL_BANDED2 too */
     GBA_KERNEL_WARP16 = 16,    /* bands of 64 strips, one warp per band, int16x2 DPX, 4-bit trace */
-    GBA_KERNEL_DYNAMIC = 32    /* DynamicGaps cells, one pair per thread */
+    GBA_KERNEL_DYNAMIC = 32,   /* DynamicGaps cells, one pair per thread */
+    GBA_KERNEL_BANDED2 = 64,   /* banded DP, two pairs of equal lengths per thread */
+    GBA_KERNEL_PIPELINED = 128,/* GBA_KERNEL_WARP16 with the bands of some pair on several warps */
+    GBA_KERNEL_ENUM_WARP = 256,/* gba_local_enumerate: a warp per pair (else a thread) */
+    GBA_KERNEL_EXTEND2 = 512   /* gba_extend_alignments: two sides per thread (else groups of lanes) */
 };
 GBA_API int gba_get_stats(gba_context *ctx, gba_stats *stats);
 

@@ -35,7 +35,8 @@ GBA_FLAG_PACKED = 32
 GBA_FLAG_PACKED_SPLIT, GBA_FLAG_PACKED_NO_SPLIT, GBA_FLAG_NO_WARP16, GBA_FLAG_WARP16 = 64, 128, 256, 512
 GBA_FLAG_XDROP = 1024
 GBA_KERNEL_STRIP, GBA_KERNEL_PACKED, GBA_KERNEL_WARP, GBA_KERNEL_BANDED, GBA_KERNEL_WARP16 = 1, 2, 4, 8, 16
-GBA_KERNEL_DYNAMIC = 32
+GBA_KERNEL_DYNAMIC, GBA_KERNEL_BANDED2, GBA_KERNEL_PIPELINED, GBA_KERNEL_ENUM_WARP, GBA_KERNEL_EXTEND2 = \
+    32, 64, 128, 256, 512
 GBA_MATCH_EXTEND, GBA_UNGAPPED_XDROP, GBA_GAPPED_XDROP = 0, 1, 2
 GBA_EXTEND_NONE, GBA_EXTEND_LEFT, GBA_EXTEND_RIGHT, GBA_EXTEND_BOTH = 0, 1, 2, 3
 

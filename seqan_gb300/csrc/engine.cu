@@ -1915,6 +1915,8 @@ int run_plan(gba_context *ctx, gba_plan *plan, const uint8_t *dseq_h, const uint
     ctx->stats.tile_rows = plan->num16 ? kVariants16[plan->variant16].rows : 0;
     ctx->stats.tile_min_blocks = plan->num16 ? kVariants16[plan->variant16].minb : 0;
     ctx->stats.dp_kernels = (plan->num16 > 0 ? GBA_KERNEL_PACKED : 0) | (plan->num_w2 > 0 ? GBA_KERNEL_WARP16 : 0) |
+                            (plan->num_w2_states > 0 ? GBA_KERNEL_PIPELINED : 0) |
+                            (plan->duo_slots > 0 ? GBA_KERNEL_BANDED2 : 0) |
                             (plan->num_slots > 0 ? (plan->params.band_on ? GBA_KERNEL_BANDED
                                                     : plan->use_warp ? GBA_KERNEL_WARP
                                                     : plan->dynamic ? GBA_KERNEL_DYNAMIC : GBA_KERNEL_STRIP)

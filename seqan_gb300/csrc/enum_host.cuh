@@ -330,6 +330,7 @@ int enumerate_impl(gba_context *ctx, const gba_enum_params *params, const int32_
     ctx->stats = gba_stats{};
     ctx->stats.dp_kernel_ms = dp_ms;
     ctx->stats.kernel_launches = launches;
+    ctx->stats.dp_kernels = warps ? GBA_KERNEL_ENUM_WARP : 0;
     ctx->stats.call_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
     return GBA_OK;
 }

@@ -498,6 +498,7 @@ int ext_paired(gba_context *ctx, const gba_extend_align_params *p, const std::ve
     ctx->stats.kernel_launches = launches + 3;
     ctx->stats.cells = int64_t(cells);
     ctx->stats.tile_rows = kX2Rows;
+    ctx->stats.dp_kernels = GBA_KERNEL_EXTEND2;
     return GBA_OK;
 }
 
