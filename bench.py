@@ -1219,12 +1219,14 @@ def run_extend_bench(args, rank, world, local_rank, dist):
     peak = C.c_double()
     ctx.check(L.gba_measure_int_peak(h, C.byref(peak)), "int peak")
     dp_ms = sum(dpk) / len(dpk)
-    passes = 1 if st.tile_rows == 16 else 2                # k_extend_dp: a score pass and a trace pass
+    paired = bool(st.dp_kernels & N.GBA_KERNEL_EXTEND2)    # two sides per thread in 16-bit halves, one pass
+    passes = 1 if paired else 2                            # k_extend_dp: a score pass and a trace pass
     ops = passes * st.cells * OPS_PER_CELL["affine_global"]
     achieved = ops / (dp_ms * 1e-3) / 1e12
     line = {"metric": "M alignments/s, batched extendAlignment (X-drop)", "value": value, "unit": "M alignments/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": kernel_ms,
-            "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
+            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+            "dtype": "int16" if paired else "int32", "data": "synthetic",
             "config": {"workload": args.workload, "description": WORKLOADS[args.workload], "alignments": n_al,
                        "cells_per_step": int(st.cells), "rows_per_band": int(st.tile_rows),
                        "value_timing": "CUDA events around the DP and the traceback inside "
@@ -1237,7 +1239,7 @@ def run_extend_bench(args, rank, world, local_rank, dist):
             "gpu_launches": args.steps * int(st.kernel_launches),
             "roofline": {"bound": "int32", "achieved": achieved, "peak": peak.value, "unit": "Tops/s",
                          "frac": achieved / peak.value if peak.value else None, "traffic": None,
-                         "kernel": "k_extend2<affine> + k_extend2_traceback" if st.tile_rows == 16 else
+                         "kernel": "k_extend2<affine> + k_extend2_traceback" if paired else
                                    "k_extend_dp<affine> (score and trace passes) + k_extend_traceback",
                          "ops_per_cell": OPS_PER_CELL["affine_global"], "dp_kernel_ms": dp_ms,
                          "gcups_per_pass": st.cells / (dp_ms / passes * 1e-3) / 1e9,
@@ -1383,7 +1385,8 @@ def run_we_bench(args, rank, world, local_rank, dist):
                           "its lanes)")
     line = {"metric": we_metric(band), "value": value,
             "unit": "pairs/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": kernel_ms,
-            "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic",
+            "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+            "dtype": "int32" if band else "int16", "data": "synthetic",
             "config": {"workload": args.workload, "description": WORKLOADS[args.workload], "pairs": n,
                        "alignments_per_step": alignments, "cells_per_step": cells,
                        "value_timing": "CUDA events around the enumeration kernel inside gba_local_enumerate "

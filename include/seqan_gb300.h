@@ -125,7 +125,9 @@ typedef struct {
  * int16 range and the batch holds at least 32768 pairs.  Other unbanded pairs whose values fit 16
  * bits (gap scores from -1024 to 0, every score between about -31,600 and 32,700) run the packed
  * 16-bit warp kernel (two strips per lane; equality scoring needs alphabet_size 1..8 there too), with
- * 16- and 32-bit score types alike; the remaining unbanded pairs run the 32-bit warp kernel.
+ * 16- and 32-bit score types alike; the remaining unbanded pairs run the 32-bit warp kernel, and so do
+ * batches of at least 16384 pairs none of which has more than 16 columns, and batches whose scratch
+ * fits hbm_budget_bytes there alone.
  * Banded pairs run one per thread, or two per thread where both have the same lengths and values of
  * 16 bits (bands of up to 40 diagonals). */
 enum {
@@ -236,7 +238,8 @@ typedef struct {
     int64_t cells;             /* algorithmic cells: sum m*n (in-band cells when banded) */
     int64_t trace_bytes;       /* trace matrix bytes written */
     int32_t tile_rows;         /* packed kernel: rows per register strip (0 = not used);
-                                  gba_extend_alignments: rows per band (8 x lanes per task) */
+                                  gba_extend_alignments: rows per band (8 x lanes per task), 16 with
+                                  two sides per thread */
     int32_t tile_min_blocks;   /* packed kernel: minimum resident blocks per SM */
     float host_plan_ms;        /* gba_align_batch: host planning time */
     float call_ms;             /* gba_align_batch: whole call, wall clock */

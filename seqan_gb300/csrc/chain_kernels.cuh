@@ -10,10 +10,10 @@
 // the trace and columns of grids too large for shared memory) in its own slice of an HBM arena.
 // Bound by the latency of a warp's own instructions: 16 warps fit an SM beside their shared memory,
 // and a grid's diagonals, tracebacks and glue follow one another.  Measured on 10,000 chains of
-// 1-3 kbp (band extension 15), whole call: 190 -> 45 ms; of a chain's 131M cycles the fill took 112M
-// before, with 28 warps on an SM, and takes 10M of 15M now with 16.  The same code runs on the host in plan mode: the grids' geometry depends only on
-// the seeds, the band extension and the sequence lengths, so a host pass sizes every chain's
-// slice before the kernel runs.
+// 1-3 kbp (band extension 15), whole call: 190 -> 47 ms; of a chain's 131M cycles the fill took 112M
+// before, with 28 warps on an SM, and takes 10M of 15M now with 16.  The same code runs on the host in
+// plan mode: the grids' geometry depends only on the seeds, the band extension and the sequence
+// lengths, so a host pass sizes every chain's slice before the kernel runs.
 //
 // Semantics followed (reference lines):
 //   chain driver          seeds/banded_chain_alignment_impl.h:660-722, 748-1330
@@ -1089,7 +1089,6 @@ struct Engine {
     // middle / bottom columns -- so values, trace bytes and init-vector stores are the loop's.  The
     // candidates for the maximum are kept per column and collected afterwards in column-major order,
     // which gives the scout's list of positions in the loop's order.
-    // Measured (10,000 chains of 1-3 kbp): whole call BEFORE -> AFTER ms.
 #ifdef __CUDA_ARCH__
     // n columns from col on, the q-th with rows r0 + q * dr0 .. r1 + q * dr1 (single: one cell);
     // p, lp: the navigator's position and leap after the previous column, advanced past the run.

@@ -15,7 +15,7 @@
 // while most of the device has nothing left to do is cut into more bands of fewer rows, which run
 // as separate tasks on different warps at the same time.
 //
-// Bound by issue to the ALU pipe in full batches (86% busy in the protein search, ncu), and by the
+// Bound by issue to the ALU pipe in full batches (85% busy in the protein search), and by the
 // latency of a lone warp's own instructions where one pair or few are in flight.  Measured, whole
 // calls, before and after this form of the kernel (rows per pair, score profile, biased values, self-
 // validating row entries, no size limits): protein search (350 residues against 20,000) 3.11 ->

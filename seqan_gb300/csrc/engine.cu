@@ -361,7 +361,8 @@ bool int16_exact(const gba_params &p, int max_pos, int64_t m, int64_t n, bool lo
 // True when the packed 16-bit warp kernel's arithmetic gives an m x n pair's exact values: every
 // value a real cell takes lies between its "infinity" and 32767.  Scores are bounded as in
 // int16_exact, with 64 columns more: a strip's lanes run on past the last column, and their halves
-// must not carry into their neighbours.  Gap scores are at most 0 (build_plan).
+// must not carry into their neighbours.  (Nor must the differences of compared values, which neighbouring
+// cells keep small whatever the substitutions: W2Input::advance.)  Gap scores are at most 0 (build_plan).
 bool w2_fits(const gba_params &p, int max_pos, int64_t m, int64_t n, bool local)
 {
     const int64_t open = -int64_t(p.gap_open), ext = -int64_t(p.gap_extend);
@@ -1166,9 +1167,9 @@ int build_plan(gba_context *ctx, const gba_params *p, const gba_batch *b, gba_pl
     // band, pipelined across warps, if that ends a fifth sooner, with fewer rows per strip (more bands
     // at once) the longer it is: the most rows whose pipeline ends within that quarter, else the rows
     // that end first.  Measured on 2,000 pairs of 100 to 10,000 bp (DP alone): an eighth 4.94 ms, a
-    // quarter 4.47, half 4.96, all of it 6.79.  The plain form pipelines bands only in batches too small to keep the GPU busy otherwise.  Row buffers: one
-    // slot of m + 1 entries for in-order pairs, two for pipelined ones; pipelined bands get a
-    // BandState each.
+    // quarter 4.47, half 4.96, all of it 6.79.  The plain form pipelines bands only in batches too small
+    // to keep the GPU busy otherwise.  Row buffers: one slot of m + 1 entries for in-order pairs, two
+    // for pipelined ones; pipelined bands get a BandState each.
     std::vector<int64_t> rb2off, bs2base;
     std::vector<int2> &w2tasks = plan->h_w2tasks;
     w2tasks.clear();
